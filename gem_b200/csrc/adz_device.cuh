@@ -87,7 +87,7 @@ __device__ __forceinline__ int coef_f32pos(double* c, int& off, float pxf, float
 
 // The cell a FP64 position selects in the reference: its FP32 rounding,
 // truncated.  Offsets stay FP64.
-__device__ __forceinline__ void cell_of(double p, int& i) { i = __double2int_rz((double)__double2float_rn(p)); }
+__device__ __forceinline__ void cell_of(double p, int& i) { i = __float2int_rz(__double2float_rn(p)); }
 
 __device__ __forceinline__ int coef_f64pos(double* c, int& off, double px8, double py8, double pz8, const DZtab& lv) {
   int ix, iy, iz;
@@ -141,17 +141,19 @@ __device__ __forceinline__ double interp1_exact(const T* __restrict__ f, const d
   return (ya[0] * c[0] + ya[2] * c[2]) + (ya[1] * c[1] + ya[3] * c[3]);
 }
 
-__device__ __forceinline__ double vmin(double a, double b) { return (a < b) ? a : b; }
-__device__ __forceinline__ double vmax(double a, double b) { return (a > b) ? a : b; }
+template <typename T>
+__device__ __forceinline__ T vmin(T a, T b) { return (a < b) ? a : b; }
+template <typename T>
+__device__ __forceinline__ T vmax(T a, T b) { return (a > b) ? a : b; }
 
 // cubic + trilinear + min/max, turbo_tricublin.c:869-997 (AVX2 box: x 1..2,
 // y 0..3, z 1..2) or the scalar 2x2x2 box (:1017-1025) when box222.
 template <typename T>
 __device__ __forceinline__ void interp_mono_exact(const T* __restrict__ f, const double* c, int ni, int ninj,
-                                                  int zlinear, bool box222, double& d, double& lin, double& mn,
-                                                  double& mx) {
+                                                  int zlinear, bool box222, double& d, double& lin, T& mn, T& mx) {
   const int ninjl = zlinear ? 0 : ninj;
-  double ya[4], mi[4], ma[4], vyl[4];
+  double ya[4], vyl[4];
+  T mi[4], ma[4];  // the bounds of values of type T
 #pragma unroll
   for (int r = 0; r < 4; r++) {
     const T* s = f + r * ni;
@@ -161,18 +163,19 @@ __device__ __forceinline__ void interp_mono_exact(const T* __restrict__ f, const
       const T* p1 = p0 + ninjl;
       const T* p2 = p1 + ninj;
       const T* p3 = p2 + ninjl;
-      const double v0 = ldd(p0), v1 = ldd(p1), v2 = ldd(p2), v3 = ldd(p3);
+      const T t1 = ldin<false>(p1), t2 = ldin<false>(p2);
+      const double v0 = ldd(p0), v1 = (double)t1, v2 = (double)t2, v3 = ldd(p3);
       double za = v0 * c[8];
       if (r == 0) {
-        mi[x] = v1;
-        ma[x] = v1;
+        mi[x] = t1;
+        ma[x] = t1;
       } else {
-        mi[x] = vmin(mi[x], v1);
-        ma[x] = vmax(ma[x], v1);
+        mi[x] = vmin(mi[x], t1);
+        ma[x] = vmax(ma[x], t1);
       }
       za = fma(v1, c[9], za);
-      mi[x] = vmin(mi[x], v2);
-      ma[x] = vmax(ma[x], v2);
+      mi[x] = vmin(mi[x], t2);
+      ma[x] = vmax(ma[x], t2);
       za = fma(v2, c[10], za);
       za = fma(v3, c[11], za);
       ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
@@ -188,11 +191,12 @@ __device__ __forceinline__ void interp_mono_exact(const T* __restrict__ f, const
   if (box222) {
     // scalar branch: start at point [1,1,1], rows 1..2, planes 1..2, x 1..2
     const int ninj2 = ninj + ninjl;
-    double a = ldd(f + 1 + ni + ninjl), lo = a, hi = a;
+    const T a = ldin<false>(f + 1 + ni + ninjl);
+    T lo = a, hi = a;
 #pragma unroll
     for (int i = 1; i < 3; i++) {
-      const double e1 = ldd(f + i + ni + ninjl), e2 = ldd(f + i + ni + ninj2);
-      const double e3 = ldd(f + i + 2 * ni + ninjl), e4 = ldd(f + i + 2 * ni + ninj2);
+      const T e1 = ldin<false>(f + i + ni + ninjl), e2 = ldin<false>(f + i + ni + ninj2);
+      const T e3 = ldin<false>(f + i + 2 * ni + ninjl), e4 = ldin<false>(f + i + 2 * ni + ninj2);
       hi = vmax(hi, e1); hi = vmax(hi, e2);
       lo = vmin(lo, e1); lo = vmin(lo, e2);
       hi = vmax(hi, e3); hi = vmax(hi, e4);

@@ -531,6 +531,10 @@ extern "C" int adzc_setup(const adzc_grid* gin, adzc_handle** out) {
   D.lminx = lminx; D.lminy = lminy;
   D.nit = I.nit; D.njt = I.njt;
   D.nij = (long long)I.nit * I.njt;
+  D.wnx = ni + 4;
+  D.wnxy = (ni + 4) * (nj + 4);
+  D.wcomp = (long long)D.wnxy * nk;
+  D.nxy = ni * nj;
   D.i0g = g.i0g; D.j0g = g.j0g;
   D.i0 = I.i0; D.in = I.in; D.j0 = I.j0; D.jn = I.jn;
   D.i0u = I.i0u; D.inu = I.inu; D.j0v = I.j0v; D.jnv = I.jnv;

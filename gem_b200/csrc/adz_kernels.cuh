@@ -116,16 +116,16 @@ struct WindLayout {
   static constexpr bool soa = (PREC == kMixed) && (ADZ_MIXED_SOA != 0);
 };
 
+// offsets into the extended, the (ni,nj,nk) and the Adz_wpxyz arrays; the
+// first two volumes are below 2^31 (adzc_setup refuses larger tiles)
 __device__ __forceinline__ long long ext_index(const DGrid& g, int i, int j, int k) {
-  return (long long)(i - g.lminx) + (long long)(j - g.lminy) * g.nit + (long long)(k - 1) * g.nij;
+  return (i - g.lminx) + (j - g.lminy) * g.nit + (k - 1) * (int)g.nij;
 }
 __device__ __forceinline__ long long arr_index(const DGrid& g, int i, int j, int k) {
-  return (long long)(i - 1) + (long long)(j - 1) * g.ni + (long long)(k - 1) * g.ni * g.nj;
+  return (i - 1) + (j - 1) * g.ni + (k - 1) * g.nxy;
 }
 __device__ __forceinline__ long long wp_index(const DGrid& g, int i, int j, int k, int c) {
-  const long long nx = g.ni + 4, ny = g.nj + 4;
-  return (long long)(i + 1) + (long long)(j + 1) * nx + (long long)(k - 1) * nx * ny +
-         (long long)(c - 1) * nx * ny * g.nk;
+  return ((i + 1) + (j + 1) * g.wnx + (k - 1) * g.wnxy) + (c - 1) * g.wcomp;
 }
 __device__ __forceinline__ double dmin_(double a, double b) { return a < b ? a : b; }
 __device__ __forceinline__ double dmax_(double a, double b) { return a > b ? a : b; }
@@ -334,6 +334,33 @@ __device__ __forceinline__ void arrival_winds(const DGrid& g, const TrajArgs& a,
   }
 }
 
+// the end of an update: departure winds (ud, vd, wd) to the new departure
+// point (xm, ym, w3) and the clipped start of the next update in (px,py,pz).
+// Returns 0 or kErrNonFinite.
+template <int PREC>
+__device__ __forceinline__ int traj_advance(const DGrid& g, const TrajArgs& a, int i, int j, int k, double ua,
+                                            double va, double wa, double ud, double vd, double wd, double& px,
+                                            double& py, double& pz, double& xm, double& ym, double& w3) {
+  const int nk = g.nk;
+  xm = (double)(i + g.i0g - 1) - (a.dt.dtD * ud + a.dt.dtA * ua) * g.inv_hx;
+  ym = (double)(j + g.j0g - 1) - (a.dt.dtD * vd + a.dt.dtA * va) * g.inv_hy;
+  const double pos = __ldg(g.zm + k) - a.dt.dtzD * wd - a.dt.dtzA * wa;
+  const double zmv = dmin_(dmax_(pos, g.zmin), g.zmax);
+  int kk1 = vsearch(zmv, g.zm, g.ovdzm, g.search_m, g.pnz_m, g.sig, nk);
+  kk1 = imin_(nk + 1, imax_(0, kk1));
+  const int nb = imax_(imin_(kk1, nk - 1), 1);
+  w3 = (zmv - __ldg(g.zm + nb)) * __ldg(g.odelz_m + nb) + (double)nb;
+  const double cx = dmin_(dmax_(xm, g.imnx), g.imxx);
+  const double cyv = dmin_(dmax_(ym, g.imny), g.imxy);
+  if (PREC == kRef32) {
+    px = (float)cx; py = (float)cyv; pz = (float)w3;
+  } else {
+    px = cx; py = cyv; pz = w3;
+  }
+  if (!isfinite(xm) || !isfinite(ym) || !isfinite(w3)) return kErrNonFinite;
+  return 0;
+}
+
 // one fixed-point update (adz_traject.F90:66-110): departure winds at
 // (px,py,pz), new departure point (xm, ym, w3) and the clipped start of the
 // next update in (px,py,pz).  Returns 0, kErrHalo or kErrNonFinite.
@@ -346,7 +373,6 @@ __device__ __forceinline__ int traj_update(const DGrid& g, const TrajArgs& a, in
   const F* __restrict__ uvw = (const F*)a.uvw_d;
   const long long e111 = ext_index(g, 1, 1, 1);
   const F* f3 = uvw + 3 * e111;
-  const int nk = g.nk;
   double ud, vd;
   int off;
   if (PREC == kMixed) {
@@ -379,23 +405,7 @@ __device__ __forceinline__ int traj_update(const DGrid& g, const TrajArgs& a, in
       ud = o[0]; vd = o[1]; wd = o[2];
     }
   }
-  xm = (double)(i + g.i0g - 1) - (a.dt.dtD * ud + a.dt.dtA * ua) * g.inv_hx;
-  ym = (double)(j + g.j0g - 1) - (a.dt.dtD * vd + a.dt.dtA * va) * g.inv_hy;
-  const double pos = __ldg(g.zm + k) - a.dt.dtzD * wd - a.dt.dtzA * wa;
-  const double zmv = dmin_(dmax_(pos, g.zmin), g.zmax);
-  int kk1 = vsearch(zmv, g.zm, g.ovdzm, g.search_m, g.pnz_m, g.sig, nk);
-  kk1 = imin_(nk + 1, imax_(0, kk1));
-  const int nb = imax_(imin_(kk1, nk - 1), 1);
-  w3 = (zmv - __ldg(g.zm + nb)) * __ldg(g.odelz_m + nb) + (double)nb;
-  const double cx = dmin_(dmax_(xm, g.imnx), g.imxx);
-  const double cyv = dmin_(dmax_(ym, g.imny), g.imxy);
-  if (PREC == kRef32) {
-    px = (float)cx; py = (float)cyv; pz = (float)w3;
-  } else {
-    px = cx; py = cyv; pz = w3;
-  }
-  if (!isfinite(xm) || !isfinite(ym) || !isfinite(w3)) return kErrNonFinite;
-  return 0;
+  return traj_advance<PREC>(g, a, i, j, k, ua, va, wa, ud, vd, wd, px, py, pz, xm, ym, w3);
 }
 
 // starting position of a warm trajectory: the stored departure point, x and y
@@ -407,9 +417,10 @@ __device__ __forceinline__ void warm_start(const DGrid& g, const TrajArgs& a, in
     const long long ar = arr_index(g, i, j, k);
     px = a.pxyzm[3 * ar]; py = a.pxyzm[3 * ar + 1]; pz = a.pxyzm[3 * ar + 2];
   } else {
-    px = dmin_(dmax_(a.wpxyz[wp_index(g, i, j, k, 1)], g.imnx), g.imxx);
-    py = dmin_(dmax_(a.wpxyz[wp_index(g, i, j, k, 2)], g.imny), g.imxy);
-    pz = a.wpxyz[wp_index(g, i, j, k, 3)];
+    const double* w = a.wpxyz + wp_index(g, i, j, k, 1);
+    px = dmin_(dmax_(w[0], g.imnx), g.imxx);
+    py = dmin_(dmax_(w[g.wcomp], g.imny), g.imxy);
+    pz = w[2 * g.wcomp];
   }
 }
 
@@ -461,9 +472,10 @@ template <int PREC>
 __device__ __forceinline__ void traj_store(const DGrid& g, const TrajArgs& a, int i, int j, int k, double xm, double ym,
                                            double w3, double px, double py, double pz, double wd) {
   using F = typename Types<PREC>::F;
-  a.wpxyz[wp_index(g, i, j, k, 1)] = xm;
-  a.wpxyz[wp_index(g, i, j, k, 2)] = ym;
-  a.wpxyz[wp_index(g, i, j, k, 3)] = w3;
+  double* w = a.wpxyz + wp_index(g, i, j, k, 1);
+  w[0] = xm;
+  w[g.wcomp] = ym;
+  w[2 * g.wcomp] = w3;
   const long long ar = arr_index(g, i, j, k);
   if (PREC == kRef32) {
     a.pxyzm[3 * ar] = (float)px;
@@ -664,54 +676,56 @@ __device__ __forceinline__ void set_position(const DGrid& g, const SetArgs& a, i
                                              double& py, double& pz) {
   using F = typename Types<PREC>::F;
   const double aa = -0.0625, bb = 0.5625, half = 0.5;
-  const double* W = a.wpxyz;
-#define WPX(ii, jj, kk, cc) ld_traj<double, CG>(W + wp_index(g, ii, jj, kk, cc))
+  const double* Wx = a.wpxyz + wp_index(g, i, j, k, 1);
+  const double* Wy = Wx + g.wcomp;
+  const double* Wz = Wy + g.wcomp;
+#define LX(o) ld_traj<double, CG>(Wx + (o))
+#define LY(o) ld_traj<double, CG>(Wy + (o))
+#define LZ(o) ld_traj<double, CG>(Wz + (o))
   if (set == 0) {
     if (PREC == kRef32) {
       const long long ar = arr_index(g, i, j, k);
       px = a.pxyzm[3 * ar]; py = a.pxyzm[3 * ar + 1]; pz = a.pxyzm[3 * ar + 2];
     } else {
-      px = dmin_(dmax_(WPX(i, j, k, 1), g.imnx), g.imxx);
-      py = dmin_(dmax_(WPX(i, j, k, 2), g.imny), g.imxy);
-      pz = WPX(i, j, k, 3);
+      px = dmin_(dmax_(LX(0), g.imnx), g.imxx);
+      py = dmin_(dmax_(LY(0), g.imny), g.imxy);
+      pz = LZ(0);
     }
     return;
   }
   if (set == 1 || set == 2) {
-    const int di = (set == 1), dj = (set == 2);
-    double c[3];
-#pragma unroll
-    for (int q = 1; q <= 3; q++)
-      c[q - 1] = aa * (WPX(i - di, j - dj, k, q) + WPX(i + 2 * di, j + 2 * dj, k, q)) +
-                 bb * (WPX(i, j, k, q) + WPX(i + di, j + dj, k, q));
-    if (set == 1) c[0] = c[0] - 0.5;
-    else c[1] = c[1] - 0.5;
-    px = dmin_(dmax_(c[0], g.imnx), g.imxx);
-    py = dmin_(dmax_(c[1], g.imny), g.imxy);
-    pz = dmin_(dmax_(c[2], 0.0), (double)(g.nk + 1));
+    const int d = set == 1 ? 1 : g.wnx;
+    double c0 = aa * (LX(-d) + LX(2 * d)) + bb * (LX(0) + LX(d));
+    double c1 = aa * (LY(-d) + LY(2 * d)) + bb * (LY(0) + LY(d));
+    const double c2 = aa * (LZ(-d) + LZ(2 * d)) + bb * (LZ(0) + LZ(d));
+    if (set == 1) c0 = c0 - 0.5;
+    else c1 = c1 - 0.5;
+    px = dmin_(dmax_(c0, g.imnx), g.imxx);
+    py = dmin_(dmax_(c1, g.imny), g.imxy);
+    pz = dmin_(dmax_(c2, 0.0), (double)(g.nk + 1));
     return;
   }
   // set T: Adz_pb
-  const F* wd = (const F*)a.wdep;
-  const F* zd = (const F*)a.zdt0;
+  const F* wd = (const F*)a.wdep + arr_index(g, i, j, k);
   const int nk = g.nk;
-  const long long e = ext_index(g, i, j, k);
-#define WD(kk) ld_traj<F, CG>(wd + arr_index(g, i, j, kk))
+  const F* zd = (const F*)a.zdt0 + ext_index(g, i, j, k);
+  const int p = g.wnxy, q = g.nxy;
+#define WD(o) ld_traj<F, CG>(wd + (o))
   double xt, yt, ztv;
   if (k >= imax_(a.k00, 2) && k <= nk - 2) {
-    const double* vw = g.vw;
-    const double w1 = __ldg(vw + 4 * (nk + 1) + k), w2 = __ldg(vw + 5 * (nk + 1) + k);
-    const double w3 = __ldg(vw + 6 * (nk + 1) + k), w4 = __ldg(vw + 7 * (nk + 1) + k);
-    xt = w1 * WPX(i, j, k - 1, 1) + w2 * WPX(i, j, k, 1) + w3 * WPX(i, j, k + 1, 1) + w4 * WPX(i, j, k + 2, 1);
-    yt = w1 * WPX(i, j, k - 1, 2) + w2 * WPX(i, j, k, 2) + w3 * WPX(i, j, k + 1, 2) + w4 * WPX(i, j, k + 2, 2);
-    const double wdt = w1 * (double)WD(k - 1) + w2 * (double)WD(k) + w3 * (double)WD(k + 1) + w4 * (double)WD(k + 2);
-    ztv = __ldg(g.zt + k) - a.dt.dtzD * wdt - a.dt.dtzA * (double)zd[e];
+    const double* vw = g.vw + 4 * (nk + 1) + k;
+    const double w1 = __ldg(vw), w2 = __ldg(vw + (nk + 1));
+    const double w3 = __ldg(vw + 2 * (nk + 1)), w4 = __ldg(vw + 3 * (nk + 1));
+    xt = w1 * LX(-p) + w2 * LX(0) + w3 * LX(p) + w4 * LX(2 * p);
+    yt = w1 * LY(-p) + w2 * LY(0) + w3 * LY(p) + w4 * LY(2 * p);
+    const double wdt = w1 * (double)WD(-q) + w2 * (double)WD(0) + w3 * (double)WD(q) + w4 * (double)WD(2 * q);
+    ztv = __ldg(g.zt + k) - a.dt.dtzD * wdt - a.dt.dtzA * (double)zd[0];
   } else if (k == nk - 1) {
-    xt = (WPX(i, j, k, 1) + WPX(i, j, k + 1, 1)) * half;
-    yt = (WPX(i, j, k, 2) + WPX(i, j, k + 1, 2)) * half;
-    const F ws = WD(k) + WD(k + 1);
+    xt = (LX(0) + LX(p)) * half;
+    yt = (LY(0) + LY(p)) * half;
+    const F ws = WD(0) + WD(q);
     const double wdt = (double)ws * half;
-    ztv = __ldg(g.zt + k) - a.dt.dtzD * wdt - a.dt.dtzA * (double)zd[e];
+    ztv = __ldg(g.zt + k) - a.dt.dtzD * wdt - a.dt.dtzA * (double)zd[0];
   } else if (k == nk) {
     if (g.slt_winds && a.uslt && a.vslt) {
       const long long a2 = (long long)(i - 1) + (long long)(j - 1) * g.ni;
@@ -719,21 +733,23 @@ __device__ __forceinline__ void set_position(const DGrid& g, const SetArgs& a, i
            g.inv_rayt * a.dt.dt * (double)((const F*)a.uslt)[a2] * __ldg(g.cy + (j - g.lminy)) * g.inv_hx;
       yt = (double)(j + g.j0g - 1) - g.inv_rayt * a.dt.dt * (double)((const F*)a.vslt)[a2] * g.inv_hy;
     } else {
-      xt = g.wp * WPX(i, j, k, 1) + g.wm * WPX(i, j, k - 1, 1);
-      yt = g.wp * WPX(i, j, k, 2) + g.wm * WPX(i, j, k - 1, 2);
+      xt = g.wp * LX(0) + g.wm * LX(-p);
+      yt = g.wp * LY(0) + g.wm * LY(-p);
     }
-    const F ws = WD(k - 1) + WD(k);
+    const F ws = WD(-q) + WD(0);
     const double wdt = (double)ws * half;
-    ztv = __ldg(g.zt + k) - g.ww * (a.dt.dtzD * wdt + a.dt.dtzA * (double)zd[e - g.nij]);
+    ztv = __ldg(g.zt + k) - g.ww * (a.dt.dtzD * wdt + a.dt.dtzA * (double)zd[-(long long)g.nij]);
   } else {  // k == 1 (k00 == 1)
-    xt = (WPX(i, j, 1, 1) + WPX(i, j, 2, 1)) * half;
-    yt = (WPX(i, j, 1, 2) + WPX(i, j, 2, 2)) * half;
-    const F ws = WD(1) + WD(2);
+    xt = (LX((1 - k) * p) + LX((2 - k) * p)) * half;
+    yt = (LY((1 - k) * p) + LY((2 - k) * p)) * half;
+    const F ws = WD((1 - k) * q) + WD((2 - k) * q);
     const double wdt = (double)ws * half;
-    ztv = __ldg(g.zt + 1) - a.dt.dtzD * wdt - a.dt.dtzA * (double)zd[e];
+    ztv = __ldg(g.zt + 1) - a.dt.dtzD * wdt - a.dt.dtzA * (double)zd[0];
   }
 #undef WD
-#undef WPX
+#undef LX
+#undef LY
+#undef LZ
   px = dmin_(dmax_(xt, g.imnx), g.imxx);
   py = dmin_(dmax_(yt, g.imny), g.imxy);
   pz = zindx_t(g, ztv);
@@ -789,9 +805,10 @@ __device__ __forceinline__ void set_point(const DGrid& g, int set, const SetArgs
     for (int q = 0; q < fp.nf; q++) {
       const F* f = (const F*)fp.src[q] + e111 + off;
       if (((fp.mono_mask >> q) & 1u) || PERT) {
-        double d, lin, mn, mx;
-        interp_mono_exact<F>(f, c, lv.ni, lv.nij, zl, fp.box222 != 0, d, lin, mn, mx);
-        F df = (F)d, lf = (F)lin, mnf = (F)mn, mxf = (F)mx;
+        double d, lin;
+        F mnf, mxf;
+        interp_mono_exact<F>(f, c, lv.ni, lv.nij, zl, fp.box222 != 0, d, lin, mnf, mxf);
+        F df = (F)d, lf = (F)lin;
         // mcrhsint perturbation in the field type (adz_interp_hlt.F90:125-133)
         if (PERT) df = df + pert_at<F>(a, i, j) * fabs_(df - lf);
         // Adz_post lin/min/max (adz_interp_hlt.F90:156-158), clip of adz_post_tr.F90:86-89
@@ -1020,12 +1037,13 @@ __global__ void __launch_bounds__(128) k_interp_pos(DZtab lv, int n, const void*
         for (int q = 0; q < fp.nf; q++) {
           const F* f = (const F*)fp.src[q] + off;
           if (KIND == 1) {
-            double d, lin, mn, mx;
+            double d, lin;
+            F mn, mx;
             interp_mono_exact<F>(f, c, lv.ni, lv.nij, zl, fp.box222 != 0, d, lin, mn, mx);
             ((F*)fp.dst[q])[o] = (F)d;
             ((F*)fp.lin[q])[o] = (F)lin;
-            ((F*)fp.mn[q])[o] = (F)mn;
-            ((F*)fp.mx[q])[o] = (F)mx;
+            ((F*)fp.mn[q])[o] = mn;
+            ((F*)fp.mx[q])[o] = mx;
           } else {
             ((F*)fp.dst[q])[o] = (F)interp1_exact<F>(f, c, lv.ni, lv.nij, zl);
           }

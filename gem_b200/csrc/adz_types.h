@@ -27,6 +27,9 @@ struct DZtab {
 struct DGrid {
   int ni, nj, nk, halox, haloy, lminx, lminy, nit, njt;
   long long nij;
+  int wnx, wnxy;      // Adz_wpxyz: row and plane lengths (ni + 4, (ni + 4)(nj + 4))
+  long long wcomp;    // and component length
+  int nxy;            // ni * nj
   int i0g, j0g;
   int i0, in, j0, jn, i0u, inu, j0v, jnv, i0b, inb, j0b, jnb, k0, k0t, k0m;
   int pnz_m, pnz_t, slt_winds, autobar;
