@@ -14,6 +14,7 @@
 #pragma once
 #include "adz_device.cuh"
 #include "adz_qv.cuh"
+#include <type_traits>
 
 // launch bounds of the gather kernels (minimum resident blocks of 128 threads
 // per SM; 0 lets ptxas choose).  A translation unit may set them before
@@ -987,6 +988,10 @@ __global__ void ADZ_QV_BOUNDS k_qv_set(DGrid g, int i0, int nx, int j0, int ny, 
 #endif
 }
 
+}  // namespace adz
+#include "adz_staged.cuh"
+namespace adz {
+
 // ---------------------------------------------------------------------------
 // explicit positions; kind 0 = cubic, 1 = mono, 2 = 3-component
 template <int PREC, int KIND>
@@ -1297,6 +1302,9 @@ cudaError_t launch_inittraj(const DGrid& g, float* pxyzm, double* wpxyz, cudaStr
 
 template <int PREC>
 cudaError_t launch_traject(const DGrid& g, const TrajArgs& a, cudaStream_t s) {
+  if constexpr (PREC != kRef32)
+    if (st_grid_ok<PREC>(g, a.k00, g.nj))
+      return st_launch_traject<PREC, false>(g, a, 1, g.ni, 1, g.nj, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
 #if ADZ_TRAJ_TILE_K > 1
   constexpr int TK = ADZ_TRAJ_TILE_K, TI = ADZ_TRAJ_TILE_I;
   const long long nb = (long long)((g.ni + TI - 1) / TI) * ((g.nk - a.k00 + 1 + TK - 1) / TK) * g.nj;
@@ -1314,6 +1322,9 @@ cudaError_t launch_traject_box(const DGrid& g, const TrajArgs& a, int i0, int nx
   const long long nkp = g.nk - a.k00 + 1, n = (long long)nx * ny * nkp;
   if (n <= 0) return cudaSuccess;
   if (batch_use_tiles(nx, nkp)) {
+    if constexpr (PREC != kRef32)
+      if (st_grid_ok<PREC>(g, a.k00, ny))
+        return st_launch_traject<PREC, false>(g, a, i0, nx, j0, ny, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
     const long long nb = (long long)((nx + 31) / 32) * ((nkp + 3) / 4) * ny;
     if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;
     k_traject_box<PREC, true><<<(unsigned)nb, 128, 0, s>>>(g, a, i0, nx, j0, ny);
@@ -1337,6 +1348,11 @@ cudaError_t launch_prepare_box(const DGrid& g, const void* uu, const void* vv, c
 template <int PREC>
 cudaError_t launch_traject_tol(const DGrid& g, const TrajArgs& a, double tol, int maxit, unsigned char* iters,
                                unsigned long long* stats, cudaStream_t s, const GuessStart& gs) {
+#ifndef ADZ_NO_ST_TOL
+  if constexpr (PREC == kMixed)
+    if (st_grid_ok<PREC>(g, a.k00, g.nj))
+      return st_launch_traject<PREC, true>(g, a, 1, g.ni, 1, g.nj, tol, maxit, iters, stats, gs, s);
+#endif
 #if ADZ_TOL_TILES
   const long long nb = (long long)((g.ni + 31) / 32) * ((g.nk - a.k00 + 1 + 3) / 4) * g.nj;
   if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;

@@ -1,0 +1,486 @@
+// The gather kernels of the step on shared-memory boxes.
+//
+// A departure point's stencil is 64 values at addresses that are consecutive
+// in x across a warp, but the points of a warp depart from two or more levels
+// (a departure point lies within a layer of its arrival level, a grid node,
+// so its cell is the one above or below almost at random).  A global gather
+// then touches several lines per request: 2.2 data-pipe wavefronts for 32
+// scalars, and that pipe bounds the direct kernels.  Here a block of
+// 32 x TJ x TK arrival points copies the box of source cells its points
+// depart from into shared memory once (cp.async) and gathers there.  Row and
+// plane pitches are multiples of the 32 banks, so lanes with different x fall
+// in different banks whatever row or plane each of them reads: one wavefront
+// per request.
+//
+// The sums are those of the direct kernels (adz_kernels.cuh), in the same
+// order, so results are the same bit for bit.  A point whose stencil leaves
+// the box (larger spreads inside one tile occur where the flow is sheared
+// over a few cells) is done by the direct code, which also reports stencils
+// outside the array.
+#pragma once
+// included by adz_kernels.cuh after the per-point code
+
+namespace adz {
+
+// ---------------------------------------------------------------------------
+// a tile of 32 x TJ x TK points, MINB resident blocks, and room for a box of
+// RP cells in x (RP a multiple of 32 four-byte or 16 eight-byte elements), BY
+// rows and BZ planes
+template <int TJ_, int TK_, int MINB_, int RP_, int BY_, int BZ_>
+struct StShape {
+  static constexpr int TJ = TJ_, TK = TK_, MINB = MINB_, RP = RP_, BY = BY_, BZ = BZ_;
+  static constexpr int NT = 32 * TJ * TK, PP = RP * BY, BOX = PP * BZ;
+};
+// trajectory.  MIXED: three component boxes per block; two updates at 1024 x
+// 1024 x 80 6.89 ms, direct 9.57 (4 x 4 points at 2 blocks 2 % slower, 4 x 2
+// points 0.5 %, 3 x 4 points 10 %, 80 registers instead of 64 3 %).  The
+// iteration to a tolerance takes 3 blocks (80 registers): the first step of a
+// run at 768 x 640 x 80 8.77 ms, 9.07 at 4 blocks, 9.65 with the direct kernel.
+// FP64: one box of interleaved (u, v, w) cells; 1024 x 512 x 80 6.01 ms,
+// direct 8.43 (2 x 4 points at 2 blocks 6.20).  REF32 stays direct: its
+// conversions to FP64 bound it either way
+template <int PREC>
+struct TrajBox;
+template <>
+struct TrajBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
+template <>
+struct TrajBox<kFp64> : StShape<3, 2, 3, 48, 8, 8> {};
+// a staged box: first cell in the extended array, extents in cells
+struct StBox {
+  int ox, oy, oz, nx, ny, nz;
+};
+
+// the cell of a position: stencil corner column and row (0-based in the
+// extended array), the level pair iz0, iz0+1 and whether z is linear there
+struct StCell {
+  int ci, cj, iz0;
+  bool zl;
+  __device__ __forceinline__ int zmin() const { return zl ? iz0 : iz0 - 1; }
+  __device__ __forceinline__ int zmax() const { return zl ? iz0 + 1 : iz0 + 2; }
+};
+
+__device__ __forceinline__ StCell st_cell(const DGrid& g, const DZtab& lv, double px, double py, double pz) {
+  int ix, iy, iz;
+  cell_of(px, ix);
+  cell_of(py, iy);
+  cell_of(pz, iz);
+  iz = imin_(imax_(iz, 1), lv.nk - 1);
+  StCell c;
+  c.ci = ix + lv.offi - 1 - g.lminx;
+  c.cj = iy + lv.offj - 1 - g.lminy;
+  c.iz0 = iz - 1;
+  c.zl = c.iz0 < 1 || c.iz0 > lv.nk - 3;
+  return c;
+}
+// the 4 x 4 columns lie in the extended array (planes always do)
+__device__ __forceinline__ bool st_inside(const DGrid& g, const StCell& c) {
+  return c.ci >= 0 && c.ci + 3 < g.nit && c.cj >= 0 && c.cj + 3 < g.njt;
+}
+// the stencil lies in the box
+template <class Cell>
+__device__ __forceinline__ bool st_in_box(const StBox& b, const Cell& c) {
+  return c.ci >= b.ox && c.ci + 4 <= b.ox + b.nx && c.cj >= b.oy && c.cj + 4 <= b.oy + b.ny && c.zmin() >= b.oz &&
+         c.zmax() < b.oz + b.nz;
+}
+
+// least and greatest stencil corner over the block's stencils (use: the
+// thread has one): minima of (ci, cj, zmin, -ci, -cj, -zmax) into red[0..5]
+// (INT_MAX before; a barrier must follow)
+template <class Cell>
+__device__ __forceinline__ void st_reduce(int* red, bool use, const Cell& c) {
+  const int big = 0x7fffffff;
+  const int m0 = __reduce_min_sync(0xffffffffu, use ? c.ci : big), m1 = __reduce_min_sync(0xffffffffu, use ? c.cj : big);
+  const int m2 = __reduce_min_sync(0xffffffffu, use ? c.zmin() : big);
+  const int m3 = __reduce_min_sync(0xffffffffu, use ? -c.ci : big);
+  const int m4 = __reduce_min_sync(0xffffffffu, use ? -c.cj : big);
+  const int m5 = __reduce_min_sync(0xffffffffu, use ? -c.zmax() : big);
+  const int lane = threadIdx.x & 31;
+  const int lo = lane == 0 ? m0 : lane == 1 ? m1 : m2, hi = lane == 3 ? m3 : lane == 4 ? m4 : m5;
+  if (lane < 6) atomicMin(red + lane, lane < 3 ? lo : hi);
+}
+
+// the box that holds every reduced stencil, or the middle of their range
+// where that is larger than a box of shape C; al: x origin a multiple of al
+// cells; empty when there is no stencil.  MARGIN: with a cell around them
+template <class C, bool MARGIN>
+__device__ __forceinline__ StBox st_box(const DGrid& g, const int* red, int al) {
+  StBox b{0, 0, 0, 0, 0, 0};
+  int x0 = red[0], y0 = red[1], z0 = red[2];
+  if (x0 == 0x7fffffff) return b;
+  int x1 = 4 - red[3], y1 = 4 - red[4], z1 = 1 - red[5];
+  if (MARGIN) {
+    x0 = imax_(x0 - 1, 0);
+    y0 = imax_(y0 - 1, 0);
+    z0 = imax_(z0 - 1, 0);
+    x1 = imin_(x1 + 1, g.nit);
+    y1 = imin_(y1 + 1, g.njt);
+    z1 = imin_(z1 + 1, g.nk);
+  }
+  b.ox = (x1 - (x0 & ~(al - 1)) > C::RP ? imax_(x0, (x0 + x1 - C::RP) / 2) : x0) & ~(al - 1);
+  b.nx = imin_(x1 - b.ox, C::RP);
+  b.oy = y1 - y0 > C::BY ? (y0 + y1 - C::BY) / 2 : y0;
+  b.ny = imin_(y1 - b.oy, C::BY);
+  b.oz = z1 - z0 > C::BZ ? (z0 + z1 - C::BZ) / 2 : z0;
+  b.nz = imin_(z1 - b.oz, C::BZ);
+  return b;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// The copies of a thread: its places in a box, the same for every array of
+// one layout.  With rows of the extended array and the box's origin on
+// 16-byte boundaries (vec) LPR lanes copy a row in 16-byte chunks, else a warp
+// copies it element by element.  A row's last chunk may run past the box into
+// the row, never past the row's end (vec implies rows of whole chunks).
+template <typename T, class C>
+struct StCopy {
+  static constexpr int CH = 16 / sizeof(T);
+  static constexpr int LPR = C::RP / CH <= 16 ? 16 : 32;   // lanes of a row (vec)
+  static constexpr int VR = C::NT / LPR, ER = C::NT / 32;  // rows of a pass
+  static constexpr int SLOTS = (C::BY * C::BZ + VR - 1) / VR;
+  static_assert(C::RP % CH == 0 && C::RP / CH <= 32, "box shape");
+  int off[SLOTS], dst[SLOTS];  // vec: source and shared offsets, dst < 0 for none
+  float inv;                   // 1 / rows of a plane
+  __device__ __forceinline__ void plan(const StBox& b, const DGrid& g, bool vec) {
+    inv = __fdividef(1.0f, (float)imax_(b.ny, 1));
+    if (!vec) return;
+    const int c = (int)(threadIdx.x % LPR) * CH, r0 = threadIdx.x / LPR, rows = c < b.nx ? b.ny * b.nz : 0;
+#pragma unroll
+    for (int t = 0; t < SLOTS; t++) {
+      const int r = r0 + t * VR;
+      // r < 256 and ny <= 16: the half keeps the product clear of the next integer
+      const int z = (int)(((float)r + 0.5f) * inv), y = r - z * b.ny;
+      off[t] = z * (int)g.nij + y * g.nit + c;
+      dst[t] = r < rows ? z * C::PP + y * C::RP + c : -1;
+    }
+  }
+  __device__ __forceinline__ void copy(T* sm, const T* __restrict__ a, const StBox& b, const DGrid& g,
+                                       bool vec) const {
+    const T* base = a + ((long long)(b.ox + b.oy * g.nit) + b.oz * g.nij);
+    if (vec) {
+#pragma unroll
+      for (int t = 0; t < SLOTS; t++)
+        if (dst[t] >= 0) cp_async<16>(sm + dst[t], base + off[t]);
+    } else {
+      const int lane = threadIdx.x & 31, rows = b.ny * b.nz;
+#pragma unroll 1
+      for (int r = threadIdx.x >> 5; r < rows; r += ER) {
+        const int z = (int)(((float)r + 0.5f) * inv), y = r - z * b.ny;
+        const T* s = base + (z * (int)g.nij + y * g.nit + lane);
+        T* d = sm + z * C::PP + y * C::RP + lane;
+#pragma unroll
+        for (int x = 0; x < C::RP; x += 32)
+          if (lane + x < b.nx) cp_async<(int)sizeof(T)>(d + x, s + x);
+      }
+    }
+  }
+};
+
+// one box of cells of three interleaved values, a row per warp at a time
+template <typename T, class C>
+__device__ __forceinline__ void st_fill3(T* sm, const T* __restrict__ a, const StBox& b, const DGrid& g, bool vec) {
+  constexpr int CH = 16 / sizeof(T);
+  const T* base = a + 3 * ((long long)(b.ox + b.oy * g.nit) + b.oz * g.nij);
+  const int lane = threadIdx.x & 31, rows = b.ny * b.nz, ne = 3 * b.nx;
+  const float inv = __fdividef(1.0f, (float)imax_(b.ny, 1));
+#pragma unroll 1
+  for (int r = threadIdx.x >> 5; r < rows; r += C::NT / 32) {
+    const int z = (int)(((float)r + 0.5f) * inv), y = r - z * b.ny;
+    const T* s = base + 3 * (z * g.nij + y * g.nit);
+    T* d = sm + 3 * (z * C::PP + y * C::RP);
+    if (vec) {
+#pragma unroll
+      for (int c = 0; c < 3 * C::RP; c += 32 * CH)
+        if (c + lane * CH < ne) cp_async<16>(d + c + lane * CH, s + c + lane * CH);
+    } else {
+      for (int c = lane; c < ne; c += 32) cp_async<(int)sizeof(T)>(d + c, s + c);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// sums over a staged box; s: the stencil corner on plane iz0, d0 and d3 the
+// offsets of the lower outer and the upper outer plane from s (those of the
+// inner planes where z is linear)
+template <int RP, int PP>
+__device__ __forceinline__ float st_interp1_mixed(const float* s, int d0, int d3, const float* cx, const float* cy,
+                                                  const float* cz) {
+  const float* p0 = s + d0;
+  const float* p1 = s;
+  const float* p3 = s + d3;
+  const float2 cz0 = f2(cz[0], cz[0]), cz1 = f2(cz[1], cz[1]);
+  const float2 cz2 = f2(cz[2], cz[2]), cz3 = f2(cz[3], cz[3]);
+  float2 ya = f2(0.f, 0.f), yb = f2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const int o = r * RP, q = o + PP;
+    float2 za = __fmul2_rn(f2(p0[o], p0[o + 1]), cz0);
+    float2 zb = __fmul2_rn(f2(p0[o + 2], p0[o + 3]), cz0);
+    za = __ffma2_rn(f2(p1[o], p1[o + 1]), cz1, za);
+    zb = __ffma2_rn(f2(p1[o + 2], p1[o + 3]), cz1, zb);
+    za = __ffma2_rn(f2(p1[q], p1[q + 1]), cz2, za);
+    zb = __ffma2_rn(f2(p1[q + 2], p1[q + 3]), cz2, zb);
+    za = __ffma2_rn(f2(p3[o], p3[o + 1]), cz3, za);
+    zb = __ffma2_rn(f2(p3[o + 2], p3[o + 3]), cz3, zb);
+    const float2 cyr = f2(cy[r], cy[r]);
+    ya = __ffma2_rn(za, cyr, ya);
+    yb = __ffma2_rn(zb, cyr, yb);
+  }
+  float2 x = __fmul2_rn(ya, f2(cx[0], cx[1]));
+  x = __ffma2_rn(yb, f2(cx[2], cx[3]), x);
+  return x.x + x.y;
+}
+
+// one component of interp3_exact, from cells of three interleaved values
+template <typename T, int RP, int PP>
+__device__ __forceinline__ double st_interp3_exact(const T* s, int d0, int d3, const double* c) {
+  const T* p0 = s + 3 * d0;
+  const T* p1 = s;
+  const T* p3 = s + 3 * d3;
+  double ya[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int o = 3 * (r * RP + x);
+      double za = (double)p0[o] * c[8];
+      za = fma((double)p1[o], c[9], za);
+      za = fma((double)p1[o + 3 * PP], c[10], za);
+      za = fma((double)p3[o], c[11], za);
+      ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
+    }
+  }
+  double x0 = ya[0] * c[0];
+  x0 = fma(ya[1], c[1], x0);
+  x0 = fma(ya[2], c[2], x0);
+  return fma(ya[3], c[3], x0);
+}
+
+// FP32 weights of coef_mixed from the offsets inside the cell
+__device__ __forceinline__ void st_weights(const DZtab& lv, int iz0, bool zl, float fx, float fy, float dz, float* cx,
+                                           float* cy, float* cz) {
+  cubic_w(fx, cx);
+  cubic_w(fy, cy);
+  if (zl) {
+    cz[0] = 0.0f;
+    cz[1] = 1.0f - dz;
+    cz[2] = dz;
+    cz[3] = 0.0f;
+  } else {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(lv.zn + 8 * iz0));
+    const float2 b = __ldg(reinterpret_cast<const float2*>(lv.zn + 8 * iz0 + 4));
+    const float t = dz;
+    const float d0 = t - a.x, d1 = t, d2 = t - 1.0f, d3 = t - a.y;
+    cz[0] = d1 * d2 * d3 * a.z;
+    cz[1] = d0 * d2 * d3 * a.w;
+    cz[2] = d0 * d1 * d3 * b.x;
+    cz[3] = d0 * d1 * d2 * b.y;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// trajectory
+struct TrajState {
+  double ua, va, wa, px, py, pz, xm, ym, w3, wd;
+};
+// one update by the direct gather, for a point whose stencil is not staged
+template <int PREC>
+__device__ __noinline__ int traj_update_direct(const DGrid* g, const TrajArgs* a, int i, int j, int k, TrajState* s) {
+  return traj_update<PREC, false>(*g, *a, i, j, k, s->ua, s->va, s->wa, s->px, s->py, s->pz, s->xm, s->ym, s->w3,
+                                    s->wd);
+}
+
+// departure winds at (px, py, pz) from the staged boxes
+template <int PREC>
+__device__ __forceinline__ void st_winds(const DGrid& g, const typename Types<PREC>::F* sm, const StBox& b,
+                                         const StCell& c, double px, double py, double pz, double& ud, double& vd,
+                                         double& wd) {
+  using F = typename Types<PREC>::F;
+  using C = TrajBox<PREC>;
+  constexpr int RP = C::RP, PP = C::PP;
+  const int d0 = c.zl ? 0 : -PP, d3 = c.zl ? PP : 2 * PP;
+  const int o = (c.iz0 - b.oz) * PP + (c.cj - b.oy) * RP + (c.ci - b.ox);
+  if constexpr (PREC == kMixed) {
+    const int ix = c.ci - g.tab_m.offi + 1 + g.lminx, iy = c.cj - g.tab_m.offj + 1 + g.lminy;
+    const float fx = (float)(px - ix), fy = (float)(py - iy), dz = (float)(pz - (c.iz0 + 1));
+    float cx[4], cy[4], cz[4];
+    st_weights(g.tab_m, c.iz0, c.zl, fx, fy, dz, cx, cy, cz);
+    const float* s = sm + o;
+    ud = st_interp1_mixed<RP, PP>(s, d0, d3, cx, cy, cz);
+    vd = st_interp1_mixed<RP, PP>(s + C::BOX, d0, d3, cx, cy, cz);
+    wd = st_interp1_mixed<RP, PP>(s + 2 * C::BOX, d0, d3, cx, cy, cz);
+  } else {
+    double cf[20];
+    int off;
+    coef_f64pos(cf, off, px, py, pz, g.tab_m);
+    const F* s = sm + 3 * o;
+    ud = st_interp3_exact<F, RP, PP>(s, d0, d3, cf);
+    vd = st_interp3_exact<F, RP, PP>(s + 1, d0, d3, cf);
+    wd = st_interp3_exact<F, RP, PP>(s + 2, d0, d3, cf);
+  }
+}
+
+// All updates of a block of 32 i x TJ j x TK k points of a box of the tile
+// (columns i0.., rows j0.., levels from a.k00).  The departure cells of the
+// first update place the box, and later updates stay in it.  A cold start's
+// points move by their whole displacement, so there the box is placed again
+// when more than 1/16 of the block's points left it.
+// TOL: the iteration to a tolerance (traject_point_tol), MIXED; its start is
+// smooth and the first update scatters the levels, so its box has a margin.
+// Else a.niter updates.
+template <int PREC, bool TOL>
+__global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MINB)
+    k_traject_st(const __grid_constant__ DGrid g, const __grid_constant__ TrajArgs a, int i0, int nx, int j0, int ny,
+                 double tol, int maxit, unsigned char* iters, unsigned long long* stats,
+                 const __grid_constant__ GuessStart gs) {
+  using F = typename Types<PREC>::F;
+  using C = TrajBox<PREC>;
+  constexpr int TK = C::TK, TJ = C::TJ, AL = 16 / sizeof(F);
+  extern __shared__ uint4 st_dyn[];
+  F* sm = reinterpret_cast<F*>(st_dyn);
+  __shared__ int red[6];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = i0 + (int)blockIdx.x * 32 + lane;
+  const int k = a.k00 + (int)blockIdx.y * TK + w % TK;
+  const int j = j0 + (int)blockIdx.z * TJ + w / TK;
+  const bool vec = g.nit % AL == 0 && ((unsigned long long)a.uvw_d & 15) == 0;
+  const bool active = i < i0 + nx && k <= g.nk && j < j0 + ny;
+  if (threadIdx.x < 6) red[threadIdx.x] = 0x7fffffff;
+  TrajState s;
+  s.xm = s.ym = s.w3 = s.wd = 0.0;
+  s.px = s.py = s.pz = s.ua = s.va = s.wa = 0.0;
+  if (active) {
+    if (a.cold) {
+      s.px = (double)(i + g.i0g - 1);
+      s.py = (double)(j + g.j0g - 1);
+      s.pz = (double)k;
+    } else if (TOL && gs.d) {
+      guess_start(g, a, gs, i, j, k, s.px, s.py, s.pz);
+    } else {
+      warm_start<PREC>(g, a, i, j, k, s.px, s.py, s.pz);
+    }
+  }
+  StBox box;
+  auto place = [&](bool use, const StCell& c) {  // place the box and start its copies
+    st_reduce(red, use, c);
+    __syncthreads();
+    box = st_box<C, TOL>(g, red, vec ? AL : 1);
+    const F* uvw = (const F*)a.uvw_d;
+    if constexpr (PREC == kMixed) {
+      StCopy<F, C> cp;
+      cp.plan(box, g, vec);
+#pragma unroll
+      for (int q = 0; q < 3; q++) cp.copy(sm + q * C::BOX, uvw + q * g.nij * g.nk, box, g, vec);
+    } else {
+      st_fill3<F, C>(sm, uvw, box, g, vec);
+    }
+    cp_async_commit();
+  };
+  StCell c = st_cell(g, g.tab_m, s.px, s.py, s.pz);
+  bool ok = active && st_inside(g, c);
+  __syncthreads();
+  place(ok, c);
+  if (active) arrival_winds<PREC>(g, a, j, k, ext_index(g, i, j, k), s.ua, s.va, s.wa);
+  cp_async_wait<0>();
+  __syncthreads();
+
+  int st = 0, used = 0, left = TOL ? maxit : a.niter;
+  bool conv = false, second = a.cold != 0;  // second: the plain iteration of a guess that did not converge
+  bool run = active && left > 0;
+  for (;;) {
+    if (run) {
+      const double qx = s.px, qy = s.py, qz = s.pz;
+      if (ok && st_in_box(box, c)) {
+        double ud, vd;
+        st_winds<PREC>(g, sm, box, c, s.px, s.py, s.pz, ud, vd, s.wd);
+        st = traj_advance<PREC>(g, a, i, j, k, s.ua, s.va, s.wa, ud, vd, s.wd, s.px, s.py, s.pz, s.xm, s.ym, s.w3);
+      } else {
+        TrajState t = s;
+        st = traj_update_direct<PREC>(&g, &a, i, j, k, &t);
+        s = t;
+      }
+      left--;
+      if (st) {
+        run = false;
+      } else {
+        used++;
+        if (TOL && fabs(s.px - qx) <= tol && fabs(s.py - qy) <= tol && fabs(s.pz - qz) <= tol) {
+          conv = true;
+          run = false;
+        } else if (left == 0) {
+          run = TOL && !second;
+          if (run) {  // fallback: plain iteration from the arrival point
+            second = true;
+            left = maxit;
+            s.px = (double)(i + g.i0g - 1);
+            s.py = (double)(j + g.j0g - 1);
+            s.pz = (double)k;
+          }
+        }
+      }
+    }
+    if (a.cold) {
+      if (!__syncthreads_or(run)) break;
+    } else if (!__any_sync(0xffffffffu, run)) {
+      break;
+    }
+    c = st_cell(g, g.tab_m, s.px, s.py, s.pz);
+    ok = run && st_inside(g, c);
+    if (a.cold && __syncthreads_count(ok && !st_in_box(box, c)) > C::NT / 16) {
+      if (threadIdx.x < 6) red[threadIdx.x] = 0x7fffffff;
+      __syncthreads();
+      place(ok, c);
+      cp_async_wait<0>();
+      __syncthreads();
+    }
+  }
+  if (TOL && active && iters)
+    iters[arr_index(g, i, j, k)] = (unsigned char)(imin_(used, 127) + ((second && !a.cold) ? 128 : 0));
+  if (active && st) raise_status(g.status, st);
+  if (active && !st && used > 0) traj_store<PREC>(g, a, i, j, k, s.xm, s.ym, s.w3, s.px, s.py, s.pz, s.wd);
+  if (TOL && stats) {
+    const unsigned cnt[3] = {(unsigned)used, (unsigned)(active && second && !a.cold), (unsigned)(active && !conv)};
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const unsigned v = __reduce_add_sync(0xffffffffu, cnt[q]);
+      if (lane == 0 && v) atomicAdd(stats + q, (unsigned long long)v);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// whether the grid of a launch fits (its y and z extents are below 65536);
+// larger tiles take the direct kernels
+template <int PREC>
+bool st_grid_ok(const DGrid& g, int k00, int ny) {
+  using C = TrajBox<PREC>;
+  return (g.nk - k00 + C::TK) / C::TK <= 65535 && (ny + C::TJ - 1) / C::TJ <= 65535;
+}
+template <int PREC, bool TOL>
+cudaError_t st_launch_traject(const DGrid& g, const TrajArgs& a, int i0, int nx, int j0, int ny, double tol, int maxit,
+                              unsigned char* iters, unsigned long long* stats, const GuessStart& gs, cudaStream_t s) {
+  using C = TrajBox<PREC>;
+  const int nkp = g.nk - a.k00 + 1;
+  if (nx <= 0 || ny <= 0 || nkp <= 0) return cudaSuccess;
+  constexpr int smem = 3 * C::BOX * (int)sizeof(typename Types<PREC>::F);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_traject_st<PREC, TOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((nx + 31) / 32, (nkp + C::TK - 1) / C::TK, (ny + C::TJ - 1) / C::TJ);
+  k_traject_st<PREC, TOL><<<grid, C::NT, smem, s>>>(g, a, i0, nx, j0, ny, tol, maxit, iters, stats, gs);
+  return cudaGetLastError();
+}
+
+}  // namespace adz
