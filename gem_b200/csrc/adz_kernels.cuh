@@ -1369,6 +1369,15 @@ cudaError_t launch_tricub_set(const DGrid& g, int set, int i0, int nx, int j0, i
                               const SetArgs& a, const FieldPtrs& fp, cudaStream_t s) {
   const long long n = (long long)nx * ny * nz;
   if (n <= 0) return cudaSuccess;
+  if constexpr (PREC != kRef32) {
+    if (!a.pert) {
+      SetParts sp{};
+      sp.n = 1;
+      sp.p[0] = SetPart{fp, set, i0, nx, j0, ny, k0, nz, 0};
+      const SetParts st = st_take_parts<PREC>(sp);
+      if (st.n > 0) return st_launch_sets<PREC>(g, a, st, s);
+    }
+  }
 #if ADZ_SET_TILE_K > 1
   constexpr int TK = ADZ_SET_TILE_K, TI = 128 / TK;
   const long long nb = (long long)((nx + TI - 1) / TI) * ((nz + TK - 1) / TK) * ny;
@@ -1392,8 +1401,18 @@ cudaError_t launch_positions(const DGrid& g, int set, int i0, int nx, int j0, in
 }
 
 template <int PREC>
-cudaError_t launch_tricub_parts(const DGrid& g, const SetArgs& a, const SetParts& sp, cudaStream_t s) {
-  if (sp.n < 1 || sp.n > kMaxParts) return cudaErrorInvalidValue;
+cudaError_t launch_tricub_parts(const DGrid& g, const SetArgs& a, const SetParts& parts, cudaStream_t s) {
+  if (parts.n < 1 || parts.n > kMaxParts) return cudaErrorInvalidValue;
+  SetParts sp = parts;
+  if constexpr (PREC != kRef32) {
+    if (!a.pert) {
+      const SetParts st = st_take_parts<PREC>(sp);
+      if (st.n > 0) {
+        const cudaError_t e = st_launch_sets<PREC>(g, a, st, s);
+        if (e != cudaSuccess || sp.n == 0) return e;
+      }
+    }
+  }
   long long most = 0;  // blocks of the largest part
   for (int q = 0; q < sp.n; q++) {
 #if ADZ_SET_TILE_K > 1

@@ -45,6 +45,24 @@ template <>
 struct TrajBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
 template <>
 struct TrajBox<kFp64> : StShape<3, 2, 3, 48, 8, 8> {};
+template <int PREC>
+struct SetBox;
+// 8 fields of set t at 1024 x 1024 x 80: 7.93 ms, direct 11.19 (rows that are
+// no multiple of 16 bytes, 1021: 10.9 and 13.4); 4 x 4 points 8.21, 4 x 2
+// points 8.59
+template <>
+struct SetBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
+// FP64, 8 fields at 1024 x 512 x 80: 7.38 ms, direct 9.08
+template <>
+struct SetBox<kFp64> : StShape<2, 4, 2, 48, 7, 11> {};
+constexpr int kStRing = 3;  // boxes in flight of the sets kernel
+// fields from which a part of a sets launch is staged: placing and filling
+// the boxes costs about what two fields gain (MIXED at 1024 x 1024 x 80, 2
+// fields: 3.44 ms staged, 3.36 direct; 5 fields 5.64 and 7.19; FP64 at 1024 x
+// 512 x 80, 2 fields: 3.14 and 2.85, 5 fields 5.07 and 5.95).  REF32 stays
+// direct: its conversions bound it (8 fields: 6.93 staged, 6.38 direct)
+constexpr int kStMinFields = 3;
+
 // a staged box: first cell in the extended array, extents in cells
 struct StBox {
   int ox, oy, oz, nx, ny, nz;
@@ -243,6 +261,72 @@ __device__ __forceinline__ float st_interp1_mixed(const float* s, int d0, int d3
   return x.x + x.y;
 }
 
+template <int RP, int PP>
+__device__ __forceinline__ void st_mono_mixed(const float* s, int d0, int d3, float fx, float fy, float dz,
+                                              const float* cx, const float* cy, const float* cz, float& d, float& lin,
+                                              float& mn, float& mx) {
+  const float* p0 = s + d0;
+  const float* p1 = s;
+  const float* p3 = s + d3;
+  const float2 cz0 = f2(cz[0], cz[0]), cz1 = f2(cz[1], cz[1]);
+  const float2 cz2 = f2(cz[2], cz[2]), cz3 = f2(cz[3], cz[3]);
+  const float2 lz0 = f2(1.0f - dz, 1.0f - dz), lz1 = f2(dz, dz);
+  float2 ya = f2(0.f, 0.f), yb = f2(0.f, 0.f), yl = f2(0.f, 0.f);
+  float lo = 3.402823466e38f, hi = -3.402823466e38f;
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    const int o = r * RP, q = o + PP;
+    const float2 a1 = f2(p1[o], p1[o + 1]), b1 = f2(p1[o + 2], p1[o + 3]);
+    const float2 a2 = f2(p1[q], p1[q + 1]), b2 = f2(p1[q + 2], p1[q + 3]);
+    float2 za = __fmul2_rn(f2(p0[o], p0[o + 1]), cz0);
+    float2 zb = __fmul2_rn(f2(p0[o + 2], p0[o + 3]), cz0);
+    za = __ffma2_rn(a1, cz1, za);
+    zb = __ffma2_rn(b1, cz1, zb);
+    za = __ffma2_rn(a2, cz2, za);
+    zb = __ffma2_rn(b2, cz2, zb);
+    za = __ffma2_rn(f2(p3[o], p3[o + 1]), cz3, za);
+    zb = __ffma2_rn(f2(p3[o + 2], p3[o + 3]), cz3, zb);
+    const float2 cyr = f2(cy[r], cy[r]);
+    ya = __ffma2_rn(za, cyr, ya);
+    yb = __ffma2_rn(zb, cyr, yb);
+    lo = fminf(lo, fminf(fminf(a1.y, b1.x), fminf(a2.y, b2.x)));
+    hi = fmaxf(hi, fmaxf(fmaxf(a1.y, b1.x), fmaxf(a2.y, b2.x)));
+    if (r == 1 || r == 2) {
+      const float2 zl = __ffma2_rn(f2(a2.y, b2.x), lz1, __fmul2_rn(f2(a1.y, b1.x), lz0));
+      const float cyl = (r == 1) ? 1.0f - fy : fy;
+      yl = __ffma2_rn(zl, f2(cyl, cyl), yl);
+    }
+  }
+  float2 x = __fmul2_rn(ya, f2(cx[0], cx[1]));
+  x = __ffma2_rn(yb, f2(cx[2], cx[3]), x);
+  d = x.x + x.y;
+  lin = fmaf(yl.y, fx, yl.x * (1.0f - fx));
+  mn = lo;
+  mx = hi;
+}
+
+// interp1_exact
+template <typename T, int RP, int PP>
+__device__ __forceinline__ double st_interp_exact(const T* s, int d0, int d3, const double* c) {
+  const T* p0 = s + d0;
+  const T* p1 = s;
+  const T* p3 = s + d3;
+  double ya[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int o = r * RP + x;
+      double za = (double)p0[o] * c[8];
+      za = fma((double)p1[o], c[9], za);
+      za = fma((double)p1[o + PP], c[10], za);
+      za = fma((double)p3[o], c[11], za);
+      ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
+    }
+  }
+  return (ya[0] * c[0] + ya[2] * c[2]) + (ya[1] * c[1] + ya[3] * c[3]);
+}
+
 // one component of interp3_exact, from cells of three interleaved values
 template <typename T, int RP, int PP>
 __device__ __forceinline__ double st_interp3_exact(const T* s, int d0, int d3, const double* c) {
@@ -266,6 +350,50 @@ __device__ __forceinline__ double st_interp3_exact(const T* s, int d0, int d3, c
   x0 = fma(ya[1], c[1], x0);
   x0 = fma(ya[2], c[2], x0);
   return fma(ya[3], c[3], x0);
+}
+
+// interp_mono_exact with the 4-row box
+template <typename T, int RP, int PP>
+__device__ __forceinline__ void st_mono_exact(const T* s, int d0, int d3, const double* c, double& d, double& lin, T& mn,
+                                              T& mx) {
+  const T* p0 = s + d0;
+  const T* p1 = s;
+  const T* p3 = s + d3;
+  double ya[4], vyl[4];
+  T mi[4], ma[4];  // the bounds of values of type T
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int o = r * RP + x;
+      const T t1 = p1[o], t2 = p1[o + PP];
+      const double v0 = (double)p0[o], v1 = (double)t1, v2 = (double)t2, v3 = (double)p3[o];
+      double za = v0 * c[8];
+      if (r == 0) {
+        mi[x] = t1;
+        ma[x] = t1;
+      } else {
+        mi[x] = vmin(mi[x], t1);
+        ma[x] = vmax(ma[x], t1);
+      }
+      za = fma(v1, c[9], za);
+      mi[x] = vmin(mi[x], t2);
+      ma[x] = vmax(ma[x], t2);
+      za = fma(v2, c[10], za);
+      za = fma(v3, c[11], za);
+      ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
+      if (r == 1 || r == 2) {
+        double vzl = v1 * c[18];
+        vzl = fma(v2, c[19], vzl);
+        vyl[x] = (r == 1) ? vzl * c[16] : fma(vzl, c[17], vyl[x]);
+      }
+    }
+  }
+  mn = vmin(mi[1], mi[2]);
+  mx = vmax(ma[1], ma[2]);
+  const double l0 = vyl[0] * c[12], l1 = vyl[1] * c[13], l2 = vyl[2] * c[14], l3 = vyl[3] * c[15];
+  lin = (l0 + l2) + (l1 + l3);
+  d = (ya[0] * c[0] + ya[2] * c[2]) + (ya[1] * c[1] + ya[3] * c[3]);
 }
 
 // FP32 weights of coef_mixed from the offsets inside the cell
@@ -461,6 +589,119 @@ __global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MI
 }
 
 // ---------------------------------------------------------------------------
+// position sets
+template <int PREC>
+__device__ __noinline__ void set_point_direct(const DGrid* g, int set, const SetArgs* a, const FieldPtrs* fp, int i,
+                                              int j, int k) {
+  set_point<PREC, false, false>(*g, set, *a, *fp, i, j, k);
+}
+
+// the fields of the position sets' parts on tiles of 32 i x TJ j x TK k
+// points, consecutive blocks taking consecutive parts (u, v, t ...).  A block's
+// fields go one after another through a ring of boxes: the copies of the next
+// two run while one is summed.
+template <int PREC>
+__global__ void __launch_bounds__(SetBox<PREC>::NT, SetBox<PREC>::MINB)
+    k_sets_st(const __grid_constant__ DGrid g, const __grid_constant__ SetArgs a, const __grid_constant__ SetParts sp) {
+  using F = typename Types<PREC>::F;
+  using C = SetBox<PREC>;
+  constexpr int TK = C::TK, TJ = C::TJ, RP = C::RP, PP = C::PP, BOX = C::BOX;
+  extern __shared__ uint4 st_dyn[];
+  F* ring = reinterpret_cast<F*>(st_dyn);
+  __shared__ int red[6];
+  const unsigned part = blockIdx.x % (unsigned)sp.n;
+  const SetPart& P = sp.p[part];
+  const FieldPtrs& fp = P.fp;
+  const DZtab& lv = (P.set == 3) ? g.tab_t : g.tab_m;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int fi = (int)(blockIdx.x / (unsigned)sp.n) * 32, fk = (int)blockIdx.y * TK, fj = (int)blockIdx.z * TJ;
+  if (fi >= P.nx || fk >= P.nz || fj >= P.ny) return;
+  const int i = P.i0 + fi + lane, k = P.k0 + fk + w % TK, j = P.j0 + fj + w / TK;
+  const bool active = fi + lane < P.nx && fk + w % TK < P.nz && fj + w / TK < P.ny;
+  constexpr int AL = 16 / sizeof(F);
+  const bool vec = P.vec != 0;
+  if (threadIdx.x < 6) red[threadIdx.x] = 0x7fffffff;
+  __syncthreads();
+  StCell c{};
+  bool in = false;
+  double px = 0.0, py = 0.0, pz = 0.0;
+  if (active) {
+    set_position<PREC, false>(g, a, P.set, i, j, k, px, py, pz);
+    c = st_cell(g, lv, px, py, pz);
+    in = st_inside(g, c);
+  }
+  st_reduce(red, in, c);
+  __syncthreads();
+  const StBox box = st_box<C, false>(g, red, vec ? AL : 1);
+  StCopy<F, C> cp;
+  cp.plan(box, g, vec);
+  // copies of field q into its slot; always one group, so that group q is
+  // field q's
+  auto copy = [&](int q, int slot) {
+    if (q < fp.nf) cp.copy(ring + slot * BOX, (const F*)fp.src[q], box, g, vec);
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int q = 0; q < kStRing - 1; q++) copy(q, q);
+  in = in && st_in_box(box, c);
+  const int o = (c.iz0 - box.oz) * PP + (c.cj - box.oy) * RP + (c.ci - box.ox);
+  const int d0 = c.zl ? 0 : -PP, d3 = c.zl ? PP : 2 * PP;
+  typename std::conditional<PREC == kMixed, float, double>::type cf[20];
+  float fx = 0.f, fy = 0.f, dz = 0.f;
+  if (in) {
+    if constexpr (PREC == kMixed) {
+      fx = (float)(px - (c.ci - lv.offi + 1 + g.lminx));
+      fy = (float)(py - (c.cj - lv.offj + 1 + g.lminy));
+      dz = (float)(pz - (c.iz0 + 1));
+      st_weights(lv, c.iz0, c.zl, fx, fy, dz, cf, cf + 4, cf + 8);
+    } else {
+      int off;
+      coef_f64pos(cf, off, px, py, pz, lv);
+    }
+  }
+  const int e = (int)ext_index(g, i, j, k);
+  int use = 0, next = kStRing - 1;
+#pragma unroll 1
+  for (int q = 0; q < fp.nf; q++) {
+    cp_async_wait<kStRing - 2>();
+    __syncthreads();  // field q has arrived, and everyone is done with the slot of the next copy
+    copy(q + kStRing - 1, next);
+    next = next == kStRing - 1 ? 0 : next + 1;
+    const F* s = ring + use * BOX + o;
+    use = use == kStRing - 1 ? 0 : use + 1;
+    if (!in) continue;
+    if constexpr (PREC == kMixed) {
+      if ((fp.mono_mask >> q) & 1u) {
+        float d, lin, mn, mx;
+        st_mono_mixed<RP, PP>(s, d0, d3, fx, fy, dz, cf, cf + 4, cf + 8, d, lin, mn, mx);
+        if ((fp.clip_mask >> q) & 1u) d = fmaxf(mn, fminf(mx, d));
+        if (fp.lin[q]) ((float*)fp.lin[q])[e] = fmaxf(mn, fminf(mx, lin));
+        if (fp.mn[q]) ((float*)fp.mn[q])[e] = mn;
+        if (fp.mx[q]) ((float*)fp.mx[q])[e] = mx;
+        ((float*)fp.dst[q])[e] = d;
+      } else {
+        ((float*)fp.dst[q])[e] = st_interp1_mixed<RP, PP>(s, d0, d3, cf, cf + 4, cf + 8);
+      }
+    } else {
+      if ((fp.mono_mask >> q) & 1u) {
+        double d, lin;
+        F mnf, mxf;
+        st_mono_exact<F, RP, PP>(s, d0, d3, cf, d, lin, mnf, mxf);
+        F df = (F)d, lf = (F)lin;
+        if ((fp.clip_mask >> q) & 1u) df = (mnf > ((mxf < df) ? mxf : df)) ? mnf : ((mxf < df) ? mxf : df);
+        if (fp.lin[q]) ((F*)fp.lin[q])[e] = (mnf > ((mxf < lf) ? mxf : lf)) ? mnf : ((mxf < lf) ? mxf : lf);
+        if (fp.mn[q]) ((F*)fp.mn[q])[e] = mnf;
+        if (fp.mx[q]) ((F*)fp.mx[q])[e] = mxf;
+        ((F*)fp.dst[q])[e] = df;
+      } else {
+        ((F*)fp.dst[q])[e] = (F)st_interp_exact<F, RP, PP>(s, d0, d3, cf);
+      }
+    }
+  }
+  if (active && !in) set_point_direct<PREC>(&g, P.set, &a, &fp, i, j, k);
+}
+
+// ---------------------------------------------------------------------------
 // whether the grid of a launch fits (its y and z extents are below 65536);
 // larger tiles take the direct kernels
 template <int PREC>
@@ -468,6 +709,30 @@ bool st_grid_ok(const DGrid& g, int k00, int ny) {
   using C = TrajBox<PREC>;
   return (g.nk - k00 + C::TK) / C::TK <= 65535 && (ny + C::TJ - 1) / C::TJ <= 65535;
 }
+// takes the parts of a sets launch that the staged kernel runs out of sp:
+// those of kStMinFields fields or more whose boxes are alike (each fills at
+// least half of the region that spans the largest; not so the boxes of a
+// band) and whose grid fits
+template <int PREC>
+SetParts st_take_parts(SetParts& sp) {
+  using C = SetBox<PREC>;
+  SetParts st{}, rest{};
+  long long nx = 0, ny = 0, nz = 0;
+  for (int q = 0; q < sp.n; q++) {
+    nx = sp.p[q].nx > nx ? sp.p[q].nx : nx;
+    ny = sp.p[q].ny > ny ? sp.p[q].ny : ny;
+    nz = sp.p[q].nz > nz ? sp.p[q].nz : nz;
+  }
+  const bool fits = (nz + C::TK - 1) / C::TK <= 65535 && (ny + C::TJ - 1) / C::TJ <= 65535;
+  for (int q = 0; q < sp.n; q++) {
+    const SetPart& P = sp.p[q];
+    if (fits && P.fp.nf >= kStMinFields && 2LL * P.nx * P.ny * P.nz >= nx * ny * nz) st.p[st.n++] = P;
+    else rest.p[rest.n++] = P;
+  }
+  sp = rest;
+  return st;
+}
+
 template <int PREC, bool TOL>
 cudaError_t st_launch_traject(const DGrid& g, const TrajArgs& a, int i0, int nx, int j0, int ny, double tol, int maxit,
                               unsigned char* iters, unsigned long long* stats, const GuessStart& gs, cudaStream_t s) {
@@ -480,6 +745,30 @@ cudaError_t st_launch_traject(const DGrid& g, const TrajArgs& a, int i0, int nx,
   if (e != cudaSuccess) return e;
   const dim3 grid((nx + 31) / 32, (nkp + C::TK - 1) / C::TK, (ny + C::TJ - 1) / C::TJ);
   k_traject_st<PREC, TOL><<<grid, C::NT, smem, s>>>(g, a, i0, nx, j0, ny, tol, maxit, iters, stats, gs);
+  return cudaGetLastError();
+}
+
+template <int PREC>
+cudaError_t st_launch_sets(const DGrid& g, const SetArgs& a, const SetParts& parts, cudaStream_t s) {
+  using C = SetBox<PREC>;
+  using F = typename Types<PREC>::F;
+  SetParts sp = parts;
+  int nx = 0, ny = 0, nz = 0;
+  for (int q = 0; q < sp.n; q++) {
+    SetPart& P = sp.p[q];
+    nx = P.nx > nx ? P.nx : nx;
+    ny = P.ny > ny ? P.ny : ny;
+    nz = P.nz > nz ? P.nz : nz;
+    bool vec = g.nit % (16 / (int)sizeof(F)) == 0;
+    for (int f = 0; f < P.fp.nf; f++) vec = vec && ((uintptr_t)P.fp.src[f] & 15) == 0;
+    P.vec = vec;
+  }
+  if (nx <= 0 || ny <= 0 || nz <= 0) return cudaSuccess;
+  constexpr int smem = kStRing * C::BOX * (int)sizeof(F);
+  const cudaError_t e = cudaFuncSetAttribute(k_sets_st<PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((nx + 31) / 32 * sp.n, (nz + C::TK - 1) / C::TK, (ny + C::TJ - 1) / C::TJ);
+  k_sets_st<PREC><<<grid, C::NT, smem, s>>>(g, a, sp);
   return cudaGetLastError();
 }
 

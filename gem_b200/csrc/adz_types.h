@@ -87,7 +87,8 @@ struct FieldPtrs {
 // the tricubic field groups of several position sets in one launch
 struct SetPart {
   FieldPtrs fp;
-  int set, i0, nx, j0, ny, k0, nz, pad;
+  int set, i0, nx, j0, ny, k0, nz;
+  int vec;  // every source array and its rows lie on 16-byte boundaries (set by the staged launch)
 };
 constexpr int kMaxParts = 8;
 struct SetParts {
