@@ -1442,6 +1442,9 @@ cudaError_t launch_qv_set(const DGrid& g, int i0, int nx, int j0, int ny, int k0
                           const FieldPtrs& fp, cudaStream_t s) {
   const long long n = (long long)nx * ny * nz;
   if (n <= 0) return cudaSuccess;
+  if constexpr (PREC == kMixed)
+    if (!a.pert && fp.nf >= kStQvMinFields && (nz + 3) / 4 <= 65535 && (ny + 1) / 2 <= 65535)
+      return st_launch_qv<PREC>(g, i0, nx, j0, ny, k0, nz, a, fp, s);
 #if ADZ_QV_TILES
   const long long nb = (long long)((nx + 31) / 32) * ((nz + 3) / 4) * ny;
   if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;

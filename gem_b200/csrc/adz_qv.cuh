@@ -17,6 +17,7 @@ struct QvCoef {
   double cx[4], cy[4], qz[6], lx[2], ly[2], lz[2];
   long long off;  // ext offset of the stencil origin (column i-1, row j-1, first plane) from (1,1,1)
   int pl[6];      // plane of each of the six vertical terms, relative to the first plane
+  int kb;         // the first plane's level, from 1
 };
 
 // PREC kRef32 takes FP32 positions (the reference's Adz_pt); the others FP64
@@ -86,6 +87,7 @@ __device__ __forceinline__ void qv_coef(const DGrid& g, double px, double py, do
     c.qz[4] = 0.0;
     c.qz[5] = 0.0;
   }
+  c.kb = kb;
   const int nc = quintic ? 1 : 0, nl = (quintic || cubic) ? 1 : 0;
   c.pl[0] = 0;
   c.pl[1] = nc;

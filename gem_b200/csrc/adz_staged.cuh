@@ -61,7 +61,7 @@ constexpr int kStRing = 3;  // boxes in flight of the sets kernel
 // fields: 3.44 ms staged, 3.36 direct; 5 fields 5.64 and 7.19; FP64 at 1024 x
 // 512 x 80, 2 fields: 3.14 and 2.85, 5 fields 5.07 and 5.95).  REF32 stays
 // direct: its conversions bound it (8 fields: 6.93 staged, 6.38 direct)
-constexpr int kStMinFields = 3;
+constexpr int kStMinFields = 3, kStQvMinFields = 2;
 
 // a staged box: first cell in the extended array, extents in cells
 struct StBox {
@@ -702,6 +702,137 @@ __global__ void __launch_bounds__(SetBox<PREC>::NT, SetBox<PREC>::MINB)
 }
 
 // ---------------------------------------------------------------------------
+// BICUBH_QV, MIXED
+// 8 fields with bounds at 640 x 600 x 80: 4.29 ms, direct 6.04 (637: 5.28 and
+// 6.48); 2 fields 1.75 and 1.97, 1 field 1.40 and 1.39
+struct QvBox : StShape<2, 4, 3, 64, 7, 12> {};
+struct QvCell {
+  int ci, cj, k0, k1;
+  __device__ __forceinline__ int zmin() const { return k0; }
+  __device__ __forceinline__ int zmax() const { return k1; }
+};
+
+// interp_qv_mixed over a staged box: s the stencil's corner, p1..p5 the
+// offsets of the planes of the vertical terms
+template <int RP>
+__device__ __forceinline__ void st_qv_mixed(const float* s, int p1, int p2, int p3, int p4, int p5, const QvCoefF& w,
+                                            float& xyz, float& li, float& mi, float& ma) {
+  const float *s1 = s + p1, *s2 = s + p2, *s3 = s + p3, *s4 = s + p4, *s5 = s + p5;
+  float dst[4], dsl[2] = {0.f, 0.f};
+  float hi = s2[1 + RP], lo = hi;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    float v[4], b2 = 0.f, b3 = 0.f, c2 = 0.f, c3 = 0.f;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const int o = i + r * RP;
+      const float t2 = s2[o], t3 = s3[o];
+      float a = s[o] * w.qz[0];
+      a = fmaf(s1[o], w.qz[1], a);
+      a = fmaf(t2, w.qz[2], a);
+      a = fmaf(t3, w.qz[3], a);
+      a = fmaf(s4[o], w.qz[4], a);
+      v[r] = fmaf(s5[o], w.qz[5], a);
+      if (r == 1) {
+        b2 = t2;
+        b3 = t3;
+      } else if (r == 2) {
+        c2 = t2;
+        c3 = t3;
+      }
+    }
+    dst[i] = fmaf(v[3], w.cy[3], fmaf(v[2], w.cy[2], fmaf(v[1], w.cy[1], v[0] * w.cy[0])));
+    if (i == 1 || i == 2) {
+      dsl[i - 1] = fmaf(fmaf(c3, w.lz[1], c2 * w.lz[0]), w.ly[1], fmaf(b3, w.lz[1], b2 * w.lz[0]) * w.ly[0]);
+      hi = fmaxf(fmaxf(hi, b2), fmaxf(b3, fmaxf(c2, c3)));
+      lo = fminf(fminf(lo, b2), fminf(b3, fminf(c2, c3)));
+    }
+  }
+  xyz = fmaf(dst[3], w.cx[3], fmaf(dst[2], w.cx[2], fmaf(dst[1], w.cx[1], dst[0] * w.cx[0])));
+  li = fmaf(dsl[1], w.lx[1], dsl[0] * w.lx[0]);
+  mi = lo;
+  ma = hi;
+}
+
+template <int PREC>
+__device__ __noinline__ void qv_point_direct(const DGrid* g, const SetArgs* a, const FieldPtrs* fp, int i, int j,
+                                             int k) {
+  qv_point<PREC, false>(*g, *a, *fp, i, j, k);
+}
+
+// the fields at the t-set positions of a region, as k_sets_st: 96 values per
+// point and field instead of 64
+template <int PREC>
+__global__ void __launch_bounds__(QvBox::NT, QvBox::MINB)
+    k_qv_st(const __grid_constant__ DGrid g, const __grid_constant__ SetArgs a, const __grid_constant__ FieldPtrs fp,
+            int i0, int nx, int j0, int ny, int k0, int nz, int vec) {
+  static_assert(PREC == kMixed, "FP32 sums");
+  using C = QvBox;
+  constexpr int TK = C::TK, TJ = C::TJ, RP = C::RP, PP = C::PP, BOX = C::BOX;
+  extern __shared__ uint4 st_dyn[];
+  float* ring = reinterpret_cast<float*>(st_dyn);
+  __shared__ int red[6];
+  const int w = threadIdx.x >> 5;
+  const int i = i0 + (int)blockIdx.x * 32 + (int)(threadIdx.x & 31), k = k0 + (int)blockIdx.y * TK + w % TK;
+  const int j = j0 + (int)blockIdx.z * TJ + w / TK;
+  const bool active = i < i0 + nx && k < k0 + nz && j < j0 + ny;
+  if (threadIdx.x < 6) red[threadIdx.x] = 0x7fffffff;
+  __syncthreads();
+  QvCell cell{};
+  QvCoefF f{};
+  bool in = false;
+  int nc = 0, nl = 0;
+  if (active) {
+    double px, py, pz;
+    set_position<PREC, false>(g, a, 3, i, j, k, px, py, pz);
+    QvCoef c;
+    qv_coef<PREC>(g, px, py, pz, c);
+    qv_to_float(c, f);
+    nc = c.pl[1];
+    nl = c.pl[2] - c.pl[1];
+    cell.ci = (int)(float)px - g.i0g - g.lminx;
+    cell.cj = (int)(float)py - g.j0g - g.lminy;
+    cell.k0 = c.kb - 1;
+    cell.k1 = cell.k0 + c.pl[5];
+    in = cell.ci >= 0 && cell.ci + 3 < g.nit && cell.cj >= 0 && cell.cj + 3 < g.njt && cell.k0 >= 0 && cell.k1 < g.nk;
+  }
+  st_reduce(red, in, cell);
+  __syncthreads();
+  const StBox box = st_box<C, false>(g, red, vec ? 4 : 1);
+  StCopy<float, C> cp;
+  cp.plan(box, g, vec != 0);
+  auto copy = [&](int q, int slot) {
+    if (q < fp.nf) cp.copy(ring + slot * BOX, (const float*)fp.src[q], box, g, vec != 0);
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int q = 0; q < kStRing - 1; q++) copy(q, q);
+  in = in && st_in_box(box, cell);
+  const int o = (cell.k0 - box.oz) * PP + (cell.cj - box.oy) * RP + (cell.ci - box.ox);
+  const int p1 = nc * PP, p2 = p1 + nl * PP, p3 = p2 + PP, p4 = p3 + nl * PP, p5 = p4 + nc * PP;
+  const int e = (int)ext_index(g, i, j, k);
+  int use = 0, next = kStRing - 1;
+#pragma unroll 1
+  for (int q = 0; q < fp.nf; q++) {
+    cp_async_wait<kStRing - 2>();
+    __syncthreads();  // field q has arrived, and everyone is done with the slot of the next copy
+    copy(q + kStRing - 1, next);
+    next = next == kStRing - 1 ? 0 : next + 1;
+    const float* s = ring + use * BOX + o;
+    use = use == kStRing - 1 ? 0 : use + 1;
+    if (!in) continue;
+    float d, lin, mn, mx;
+    st_qv_mixed<RP>(s, p1, p2, p3, p4, p5, f, d, lin, mn, mx);
+    if ((fp.clip_mask >> q) & 1u) d = fmaxf(mn, fminf(mx, d));
+    if (fp.lin[q]) ((float*)fp.lin[q])[e] = fmaxf(mn, fminf(mx, lin));
+    if (fp.mn[q]) ((float*)fp.mn[q])[e] = mn;
+    if (fp.mx[q]) ((float*)fp.mx[q])[e] = mx;
+    ((float*)fp.dst[q])[e] = d;
+  }
+  if (active && !in) qv_point_direct<PREC>(&g, &a, &fp, i, j, k);
+}
+
+// ---------------------------------------------------------------------------
 // whether the grid of a launch fits (its y and z extents are below 65536);
 // larger tiles take the direct kernels
 template <int PREC>
@@ -769,6 +900,20 @@ cudaError_t st_launch_sets(const DGrid& g, const SetArgs& a, const SetParts& par
   if (e != cudaSuccess) return e;
   const dim3 grid((nx + 31) / 32 * sp.n, (nz + C::TK - 1) / C::TK, (ny + C::TJ - 1) / C::TJ);
   k_sets_st<PREC><<<grid, C::NT, smem, s>>>(g, a, sp);
+  return cudaGetLastError();
+}
+
+template <int PREC>
+cudaError_t st_launch_qv(const DGrid& g, int i0, int nx, int j0, int ny, int k0, int nz, const SetArgs& a,
+                         const FieldPtrs& fp, cudaStream_t s) {
+  using C = QvBox;
+  bool vec = g.nit % 4 == 0;
+  for (int f = 0; f < fp.nf; f++) vec = vec && ((uintptr_t)fp.src[f] & 15) == 0;
+  constexpr int smem = kStRing * C::BOX * (int)sizeof(float);
+  const cudaError_t e = cudaFuncSetAttribute(k_qv_st<PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((nx + 31) / 32, (nz + C::TK - 1) / C::TK, (ny + C::TJ - 1) / C::TJ);
+  k_qv_st<PREC><<<grid, C::NT, smem, s>>>(g, a, fp, i0, nx, j0, ny, k0, nz, vec);
   return cudaGetLastError();
 }
 
