@@ -1,0 +1,128 @@
+"""The step's gather kernels on shared-memory boxes against the direct ones,
+bit for bit (they form the same sums in the same order): trajectories against
+the phased batch plan, the position sets and BICUBH_QV against the same call
+with a zero perturbation pattern, which the direct kernels run.  Sizes at the
+edges of tiles and boxes, rows that are not 16-byte multiples, sources off a
+16-byte boundary, few levels, and flows so scattered that stencils leave their
+box or the boxes are placed more than once."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(33, 9, 5), (64, 40, 24), (97, 51, 13), (40, 41, 4), (31, 2, 8)]
+
+
+def _case(prec_name, size, wild, ntr, seed=3):
+    from gem_b200 import adz as A, synth
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    prec = A.PREC_NAMES[prec_name]
+    ft = A._field_dtype(prec)
+    cfg = synth.config_small(*size)
+    cfg.ntracers, cfg.tracer_kind = ntr, "lognormal"
+    inp = synth.make_inputs(cfg, device="cuda", dtype=ft)
+    if wild:  # departure points anywhere within the halo, levels away
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        for key, amp in (("uu_ext", 2.5 * cfg.dx), ("vv_ext", 2.5 * cfg.dx), ("ww_ext", 1500.0), ("ut0", 2.5 * cfg.dx),
+                         ("vt0", 2.5 * cfg.dx), ("zdt0", 1500.0)):
+            r = torch.rand(inp[key].shape, generator=g, device="cuda", dtype=torch.float64)
+            inp[key] = ((2.0 * r - 1.0) * amp / cfg.dt).to(ft)
+    return A, cfg, prec, ft, inp
+
+
+def _bits(t):
+    return t.contiguous().view(torch.int32 if t.dtype == torch.float32 else torch.int64)
+
+
+# niter 6 from the arrival points is the cold start
+@pytest.mark.parametrize("cold", [False, True])
+@pytest.mark.parametrize("wild", [False, True])
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("prec_name", ["mixed", "fp64"])
+def test_staged_step_equals_direct(prec_name, size, wild, cold):
+    A, cfg, prec, ft, inp = _case(prec_name, size, wild, 4)
+    srcs = [inp["src_u"], inp["src_v"], inp["src_w"]] + inp["tracers"]
+    mono = [0, 0, 0, 1, 0, 2, 1]
+    nf = [0, 1, 1, len(srcs) - 2]
+    new = lambda: [torch.full(s.shape, -7.0, dtype=ft, device="cuda") for s in srcs]  # noqa: E731
+    # direct: one phased batch step, warm from the given departure points
+    ad = A.Adz.from_config(cfg, lam=False)
+    _, wp = ad.new_state(prec)
+    ad.adz_inittraj(prec, None, wp)
+    arrival = wp.clone()
+    ad.adz_traject(prec, cfg.dt, inp, None, wp)
+    start = arrival if cold else wp
+    wp_d, out_d = start.clone(), new()
+    b = A.Batch(prec, [dict(adz=ad, dt=cfg.dt, winds=inp, wpxyz=wp_d, nfields=nf, srcs=srcs, dsts=out_d, mono=mono,
+                            niter=6 if cold else 2)])
+    b.select(8, A.Batch.PHASED)
+    b.step()
+    torch.cuda.synchronize()
+    # staged
+    ad2 = A.Adz.from_config(cfg, lam=False)
+    wp_s, out_s = start.clone(), new()
+    if cold:
+        ad2.adz_inittraj(prec, None, wp_s)
+    ad2.adz_traject(prec, cfg.dt, inp, None, wp_s, niter=0 if cold else 2)
+    ad2.adz_tricub_sets(prec, nf, srcs, out_s, mono)
+    torch.cuda.synchronize()
+    assert b.status() == ad2.status()
+    assert torch.equal(_bits(wp_s), _bits(wp_d))
+    for x, y in zip(out_s, out_d):
+        assert torch.equal(_bits(x), _bits(y))
+
+
+@pytest.mark.parametrize("offset", [0, 1])  # elements of the sources past a 16-byte boundary
+@pytest.mark.parametrize("wild", [False, True])
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("prec_name,qv,n", [("mixed", False, 3), ("mixed", False, 17), ("fp64", False, 4),
+                                            ("mixed", True, 2), ("mixed", True, 3)])
+def test_staged_sets_equal_direct(prec_name, qv, n, size, wild, offset):
+    A, cfg, prec, ft, inp = _case(prec_name, size, wild, n)
+    ad = A.Adz.from_config(cfg, lam=False)
+    _, wp = ad.new_state(prec)
+    ad.adz_inittraj(prec, None, wp)
+    ad.adz_traject(prec, cfg.dt, inp, None, wp)
+    shp = ad.ext_shape
+    srcs = []
+    for t in inp["tracers"]:
+        v = torch.empty(t.numel() + offset, dtype=ft, device="cuda")[offset:].view(shp)
+        srcs.append(v.copy_(t))
+    srcs[0][0, 1, 2] = srcs[0][shp[0] // 2, 5, 6] = srcs[0][-1, -2, -1] = float("nan")
+    mono = [(A.QV if qv else 0) | ((1, 0, 2)[q % 3] if not qv else 1 + q % 2) for q in range(n)]
+    res = []
+    for pert in (None, torch.zeros((cfg.nj, cfg.ni), dtype=ft, device="cuda")):
+        new = lambda: [torch.full(shp, -7.0, dtype=ft, device="cuda") for _ in srcs]  # noqa: E731
+        out, post = new(), (new(), new(), new())
+        ad.set_rhs_perturbation(pert)
+        ad.adz_tricub_hlt(prec, A.SET_T, srcs, out, mono=mono, post=post)
+        torch.cuda.synchronize()
+        res.append(out + [t for p in post for t in p])
+    assert ad.status() == 0
+    for x, y in zip(*res):  # by value: d + 0 * |d - lin| is d up to the sign of a zero
+        assert np.array_equal(x.cpu().numpy(), y.cpu().numpy(), equal_nan=True)
+
+
+def test_boundary_flux_shared_and_many():
+    """More tracers than one launch takes, one of them in its own flux array."""
+    A, cfg, prec, ft, inp = _case("mixed", (56, 44, 12), False, 11)
+    ad = A.Adz.from_config(cfg)
+    _, wp = ad.new_state(prec)
+    ad.adz_inittraj(prec, None, wp)
+    ad.adz_traject(prec, cfg.dt, inp, None, wp)
+    new = lambda: [torch.zeros(ad.ext_shape, dtype=ft, device="cuda") for _ in inp["tracers"]]  # noqa: E731
+    fo, fi = new(), new()
+    ad.bc_lam_flux(prec, inp["tracers"], fo, fi)
+    # tracer 2 read from the array that receives its outflow
+    go, gi = new(), new()
+    own = inp["tracers"][2].clone()
+    srcs = list(inp["tracers"])
+    srcs[2] = go[2] = own
+    m = ad.range_mask(A.SET_B, device="cuda")
+    ad.bc_lam_flux(prec, srcs, go, gi)
+    torch.cuda.synchronize()
+    assert ad.status() == 0 and float(fi[0].abs().max()) > 0 and float(fo[0].abs().max()) > 0
+    for q in range(len(srcs)):
+        assert torch.equal(fo[q][m], go[q][m]) and torch.equal(fi[q][m], gi[q][m])
