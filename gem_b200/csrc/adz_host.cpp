@@ -907,33 +907,43 @@ extern "C" int adzc_bc_lam_flux(adzc_handle* h, int prec, int ntr, const void* c
                 h->g.pil_w, h->g.pil_e, h->g.pil_s, h->g.pil_n, I.k0t, I.i0b, I.inb, I.j0b, I.jnb, h->g.maxcfl + 1};
   const int nxb = I.inb - I.i0b + 1, nyb = I.jnb - I.j0b + 1;
   if (nxb <= 0 || nyb <= 0) return ADZC_OK;
-  const size_t fb = prec == ADZC_FP64 ? sizeof(double) : sizeof(float);
-  const size_t ext = (size_t)D.nij * D.nk * fb;
-  constexpr int kChunk = adz::kMaxFields / 2;  // tracers per interpolation launch (out and in fields)
-  void* scratch = nullptr;
-  if (adz_internal_aux(h, 2 * std::min(kChunk, ntr) * ext, &scratch) != ADZC_OK) return fail(ADZC_ERR_ALLOC);
   adz::SetArgs a = set_args(h);
   a.pert = nullptr;  // the fluxes are plain interpolations (tricublin_zyx1_m_n)
   const cudaStream_t s = (cudaStream_t)stream;
-  for (int q0 = 0; q0 < ntr; q0 += kChunk) {
-    const int nf = std::min(kChunk, ntr - q0);
-    adz::FieldPtrs fp{};
-    fp.nf = 2 * nf;
-    for (int q = 0; q < nf; q++) {
-      char* mo = (char*)scratch + (size_t)(2 * q) * ext;
-      char* mi = (char*)scratch + (size_t)(2 * q + 1) * ext;
-      ADZ_CK(prec == ADZC_FP64 ? adz::launch_bc_mask<double>(m, srcs[q0 + q], mo, mi, s)
-                               : adz::launch_bc_mask<float>(m, srcs[q0 + q], mo, mi, s));
-      fp.src[2 * q] = mo;
-      fp.src[2 * q + 1] = mi;
-      fp.dst[2 * q] = fo[q0 + q];
-      fp.dst[2 * q + 1] = fi[q0 + q];
+  for (int q0 = 0; q0 < ntr; q0 += adz::kMaxFields / 2) {
+    adz::FluxPtrs fp{};
+    fp.n = std::min(adz::kMaxFields / 2, ntr - q0);
+    for (int q = 0; q < fp.n; q++) {
+      fp.src[q] = srcs[q0 + q];
+      fp.fo[q] = fo[q0 + q];
+      fp.fi[q] = fi[q0 + q];
     }
-    // Adz_pb over (i0b:inb, j0b:jnb, 1:nk): the set-t positions of those points
-    ADZ_CK(dispatch_set(prec, D, ADZC_SET_T, I.i0b, nxb, I.j0b, nyb, 1, D.nk, a, fp, s));
-    for (int q = 0; q < nf; q++)
-      ADZ_CK(prec == ADZC_FP64 ? adz::launch_bc_zero<double>(m, fo[q0 + q], fi[q0 + q], s)
-                               : adz::launch_bc_zero<float>(m, fo[q0 + q], fi[q0 + q], s));
+    // a tracer that shares memory with a flux array of its group is read from a copy
+    const size_t ext = (size_t)D.nij * D.nk * field_bytes(prec);
+    auto shares = [&](const void* p) {
+      for (int r = 0; p && r < fp.n; r++)
+        for (const void* o : {(const void*)fp.fo[r], (const void*)fp.fi[r]})
+          if ((const char*)p < (const char*)o + ext && (const char*)o < (const char*)p + ext) return true;
+      return false;
+    };
+    size_t ncopy = 0;
+    for (int q = 0; q < fp.n; q++) ncopy += shares(fp.src[q]);
+    const size_t nlist = 1 + (size_t)nxb * nyb * D.nk;
+    void* scratch = nullptr;
+    if (adz_internal_aux(h, ncopy * ext + nlist * sizeof(int), &scratch) != ADZC_OK) return fail(ADZC_ERR_ALLOC);
+    char* c = (char*)scratch;
+    for (int q = 0; ncopy > 0 && q < fp.n; q++)
+      if (shares(fp.src[q])) {
+        ADZ_CK(cudaMemcpyAsync(c, fp.src[q], ext, cudaMemcpyDeviceToDevice, s));
+        fp.src[q] = c;
+        c += ext;
+      }
+    int* list = (int*)c;
+    switch (prec) {
+      case ADZC_REF32: ADZ_CK(adz::launch_bc_flux<adz::kRef32>(D, a, m, fp, list, s)); break;
+      case ADZC_FP64: ADZ_CK(adz::launch_bc_flux<adz::kFp64>(D, a, m, fp, list, s)); break;
+      default: ADZ_CK(adz::launch_bc_flux<adz::kMixed>(D, a, m, fp, list, s)); break;
+    }
   }
   return ADZC_OK;
 }

@@ -993,6 +993,211 @@ __global__ void ADZ_QV_BOUNDS k_qv_set(DGrid g, int i0, int nx, int j0, int ny, 
 namespace adz {
 
 // ---------------------------------------------------------------------------
+// LAM boundary fluxes (B/adz_BC_LAM_Aranami_hlt.F90:18-236): FLUX_out is the
+// tracer of the core, FLUX_in that of the rest of the domain, interpolated at
+// the t-set positions of range b; FLUX_out is zero on the core, FLUX_in on
+// the pilot zones and above k0t.  The masks are functions of the global
+// position, so a stencil value is selected where it is read (0 outside its
+// mask) and no masked copy of the tracer is made.  Almost every point is a
+// core point whose stencil lies in the core, where both are 0: it costs its
+// position and two stores per tracer.
+__device__ __forceinline__ bool bc_core_x(const BcMask& m, int i) {
+  return (!m.west || i >= 1 + m.pil_w) && (!m.east || i <= m.ni - m.pil_e);
+}
+__device__ __forceinline__ bool bc_core_y(const BcMask& m, int j) {
+  return (!m.south || j >= 1 + m.pil_s) && (!m.north || j <= m.nj - m.pil_n);
+}
+__device__ __forceinline__ bool bc_dom_x(const BcMask& m, int i) {
+  return (!m.west || i >= 1) && (!m.east || i <= m.ni);
+}
+__device__ __forceinline__ bool bc_dom_y(const BcMask& m, int j) {
+  return (!m.south || j >= 1) && (!m.north || j <= m.nj);
+}
+// bits x (or r, or p) of the stencil's columns (rows, planes) in the core and
+// in the domain
+struct BcBits {
+  unsigned cx, cy, cz, dx, dy;
+  __device__ __forceinline__ bool core(int p, int r, int x) const {
+    return ((cx & dx) >> x) & ((cy & dy) >> r) & (cz >> p) & 1u;
+  }
+  __device__ __forceinline__ bool rest(int p, int r, int x) const {
+    return ((dx >> x) & (dy >> r) & 1u) && !(((cx >> x) & (cy >> r) & (cz >> p)) & 1u);
+  }
+};
+
+// interp1_mixed / interp1_exact over values that ld(p, r, x) gives
+template <typename L>
+__device__ __forceinline__ float interp1_mixed_of(L&& ld, const WF& w) {
+  const float2 cz0 = f2(w.cz[0], w.cz[0]), cz1 = f2(w.cz[1], w.cz[1]);
+  const float2 cz2 = f2(w.cz[2], w.cz[2]), cz3 = f2(w.cz[3], w.cz[3]);
+  float2 ya = f2(0.f, 0.f), yb = f2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    float2 za = __fmul2_rn(f2(ld(0, r, 0), ld(0, r, 1)), cz0), zb = __fmul2_rn(f2(ld(0, r, 2), ld(0, r, 3)), cz0);
+    za = __ffma2_rn(f2(ld(1, r, 0), ld(1, r, 1)), cz1, za);
+    zb = __ffma2_rn(f2(ld(1, r, 2), ld(1, r, 3)), cz1, zb);
+    za = __ffma2_rn(f2(ld(2, r, 0), ld(2, r, 1)), cz2, za);
+    zb = __ffma2_rn(f2(ld(2, r, 2), ld(2, r, 3)), cz2, zb);
+    za = __ffma2_rn(f2(ld(3, r, 0), ld(3, r, 1)), cz3, za);
+    zb = __ffma2_rn(f2(ld(3, r, 2), ld(3, r, 3)), cz3, zb);
+    const float2 cyr = f2(w.cy[r], w.cy[r]);
+    ya = __ffma2_rn(za, cyr, ya);
+    yb = __ffma2_rn(zb, cyr, yb);
+  }
+  float2 x = __fmul2_rn(ya, f2(w.cx[0], w.cx[1]));
+  x = __ffma2_rn(yb, f2(w.cx[2], w.cx[3]), x);
+  return x.x + x.y;
+}
+template <typename L>
+__device__ __forceinline__ double interp1_exact_of(L&& ld, const double* c) {
+  double ya[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      double za = (double)ld(0, r, x) * c[8];
+      za = fma((double)ld(1, r, x), c[9], za);
+      za = fma((double)ld(2, r, x), c[10], za);
+      za = fma((double)ld(3, r, x), c[11], za);
+      ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
+    }
+  }
+  return (ya[0] * c[0] + ya[2] * c[2]) + (ya[1] * c[1] + ya[3] * c[3]);
+}
+
+// where the fluxes of a point are zero whatever the tracer is
+__device__ __forceinline__ bool bc_zero_out(const BcMask& m, int i, int j, int k) {
+  return k >= m.k0t && j >= 1 + m.pil_s && j <= m.nj - m.pil_n && i >= 1 + m.pil_w && i <= m.ni - m.pil_e;
+}
+__device__ __forceinline__ bool bc_zero_in(const BcMask& m, bool in_b, int i, int j, int k) {
+  return k >= m.k0t ? (m.north && j >= m.nj - m.pil_n + 1) || (m.east && i >= m.ni - m.pil_e + 1) ||
+                          (m.south && j <= m.pil_s) || (m.west && i <= m.pil_w)
+                    : in_b;
+}
+
+// the fluxes of a point of range b whose stencil crosses the core's edge.
+// Almost every such point has one flux to sum (the other is zero there).
+template <int PREC>
+__device__ __forceinline__ void bc_flux_edge(const DGrid& g, const SetArgs& a, const BcMask& m, const FluxPtrs& fp,
+                                             int i, int j, int k) {
+  using F = typename Types<PREC>::F;
+  const bool zero_o = bc_zero_out(m, i, j, k), zero_i = bc_zero_in(m, true, i, j, k);
+  const int e = (int)ext_index(g, i, j, k), e111 = (int)ext_index(g, 1, 1, 1);
+  double px, py, pz;
+  set_position<PREC, false>(g, a, 3, i, j, k, px, py, pz);
+  int off = 0;
+  WF w{};
+  double c[20];
+  bool zl = false;
+  if constexpr (PREC == kMixed) {
+    coef_mixed(w, px, py, pz, g.tab_t);
+    off = w.off;
+    zl = w.zl != 0;
+  } else {
+    if (PREC == kRef32) zl = coef_f32pos(c, off, (float)px, (float)py, (float)pz, g.tab_t) != 0;
+    else zl = coef_f64pos(c, off, px, py, pz, g.tab_t) != 0;
+  }
+  const bool ok = stencil_ok(g, off);
+  BcBits bits{};
+  if (!ok) {
+    raise_status(g.status, kErrHalo);
+  } else {
+    // the stencil's corner, in local points (k from 1)
+    const int o = off + e111, ck = o / (int)g.nij, r = o - ck * (int)g.nij, cj = r / g.nit, ci = r - cj * g.nit;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int x = ci + q + g.lminx, y = cj + q + g.lminy, z = 1 + ck + (zl ? q / 2 : q);
+      bits.cx |= (unsigned)bc_core_x(m, x) << q;
+      bits.cy |= (unsigned)bc_core_y(m, y) << q;
+      bits.cz |= (unsigned)(z >= m.k0t) << q;
+      bits.dx |= (unsigned)bc_dom_x(m, x) << q;
+      bits.dy |= (unsigned)bc_dom_y(m, y) << q;
+    }
+  }
+  const int nin = g.tab_t.ni, nij = g.tab_t.nij, nl = zl ? 0 : nij;
+  for (int q = 0; q < fp.n; q++) {
+    const F* s = (const F*)fp.src[q];  // NULL: the masks themselves (PSADJ)
+    F* fo = (F*)fp.fo[q];
+    F* fi = (F*)fp.fi[q];
+    if (zero_o) fo[e] = (F)0;
+    if (zero_i) fi[e] = (F)0;
+    // flux 0 out, 1 in
+    for (int in = zero_o ? 1 : 0; ok && in < (zero_i ? 1 : 2); in++) {
+      auto ld = [&](int p, int r, int x) {
+        const F v = s ? ldin<false>(s + e111 + off + r * nin + x + (p > 0 ? nl : 0) + (p > 1 ? nij : 0) + (p > 2 ? nl : 0))
+                      : (F)1;
+        return (in ? bits.rest(p, r, x) : bits.core(p, r, x)) ? v : (F)0;
+      };
+      F v;
+      if constexpr (PREC == kMixed) v = interp1_mixed_of(ld, w);
+      else v = (F)interp1_exact_of(ld, c);
+      (in ? fi : fo)[e] = v;
+    }
+  }
+}
+
+// every point: the zeros, and the list (count, then linear indices) of the
+// points of range b that have a flux to sum.  Summing them here made warps
+// wait for their few edge points: 2.6 ms for 4 tracers at 640 x 600 x 80
+template <int PREC>
+__global__ void __launch_bounds__(128) k_bc_flux(const __grid_constant__ DGrid g, const __grid_constant__ SetArgs a,
+                                                 const __grid_constant__ BcMask m, const __grid_constant__ FluxPtrs fp,
+                                                 int* __restrict__ list) {
+  using F = typename Types<PREC>::F;
+  // one tile of 32 i by 4 levels per block
+  const unsigned nic = (unsigned)(m.ni + 31) / 32, nkg = (unsigned)(m.nk + 3) / 4;
+  const unsigned b = blockIdx.x, bj = b / nic;
+  const int lane = (int)(threadIdx.x % 32);
+  const int i = (int)(b - bj * nic) * 32 + lane + 1;
+  const int k = (int)(bj % nkg) * 4 + (int)(threadIdx.x / 32) + 1;
+  const int j = (int)(bj / nkg) + 1;
+  bool edge = false;
+  if (i <= m.ni && k <= m.nk) {
+    const bool in_b = i >= m.i0b && i <= m.inb && j >= m.j0b && j <= m.jnb;
+    const bool zero_o = bc_zero_out(m, i, j, k);
+    bool zero_i = bc_zero_in(m, in_b, i, j, k);
+    if (in_b) {
+      edge = true;
+      if (zero_o) {
+        double px, py, pz;
+        set_position<PREC, false>(g, a, 3, i, j, k, px, py, pz);
+        const StCell c = st_cell(g, g.tab_t, px, py, pz);
+        const int x = c.ci + g.lminx, y = c.cj + g.lminy;
+        // no stencil value outside the core: both fluxes are zero
+        edge = !(st_inside(g, c) && bc_core_x(m, x) && bc_core_x(m, x + 3) && bc_core_y(m, y) &&
+                 bc_core_y(m, y + 3) && bc_dom_x(m, x) && bc_dom_x(m, x + 3) && bc_dom_y(m, y) &&
+                 bc_dom_y(m, y + 3) && c.zmin() + 1 >= m.k0t);
+      }
+      zero_i = true;
+    }
+    if (!edge) {
+      const int e = (int)ext_index(g, i, j, k);
+      for (int q = 0; q < fp.n; q++) {
+        if (zero_o) ((F*)fp.fo[q])[e] = (F)0;
+        if (zero_i) ((F*)fp.fi[q])[e] = (F)0;
+      }
+    }
+  }
+  const unsigned who = __ballot_sync(0xffffffffu, edge);
+  if (who == 0) return;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(list, __popc(who));
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(who & ((1u << lane) - 1));
+  if (edge) list[1 + at] = (i - 1) + (j - 1) * m.ni + (k - 1) * m.ni * m.nj;
+}
+
+template <int PREC>
+__global__ void __launch_bounds__(128) k_bc_edge(const __grid_constant__ DGrid g, const __grid_constant__ SetArgs a,
+                                                 const __grid_constant__ BcMask m, const __grid_constant__ FluxPtrs fp,
+                                                 const int* __restrict__ list) {
+  const int n = list[0];
+  for (int t = blockIdx.x * 128 + (int)threadIdx.x; t < n; t += gridDim.x * 128) {
+    const int p = list[1 + t], r = p / m.ni;
+    bc_flux_edge<PREC>(g, a, m, fp, p - r * m.ni + 1, r % m.nj + 1, r / m.nj + 1);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // explicit positions; kind 0 = cubic, 1 = mono, 2 = 3-component
 template <int PREC, int KIND>
 __global__ void __launch_bounds__(128) k_interp_pos(DZtab lv, int n, const void* __restrict__ pos, FieldPtrs fp) {
@@ -1458,6 +1663,20 @@ cudaError_t launch_qv_set(const DGrid& g, int i0, int nx, int j0, int ny, int k0
 }
 
 template <int PREC>
+cudaError_t launch_bc_flux(const DGrid& g, const SetArgs& a, const BcMask& m, const FluxPtrs& fp, int* list,
+                           cudaStream_t s) {
+  const long long nb = (long long)((m.ni + 31) / 32) * ((m.nk + 3) / 4) * m.nj;
+  if (nb <= 0 || fp.n <= 0) return cudaSuccess;
+  if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const cudaError_t e = cudaMemsetAsync(list, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  k_bc_flux<PREC><<<(unsigned)nb, 128, 0, s>>>(g, a, m, fp, list);
+  const long long most = (long long)(m.inb - m.i0b + 1) * (m.jnb - m.j0b + 1) * m.nk;
+  k_bc_edge<PREC><<<grid_for(most, 128, 148 * 8), 128, 0, s>>>(g, a, m, fp, list);
+  return cudaGetLastError();
+}
+
+template <int PREC>
 cudaError_t launch_interp_pos(const DZtab& lv, int kind, int n, const void* pos, const FieldPtrs& fp,
                               cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
@@ -1538,6 +1757,8 @@ int batch_resident_blocks(int variant) {
 
 #define ADZ_INSTANTIATE(P)                                                                                         \
   template cudaError_t launch_prepare<P>(const DGrid&, const void*, const void*, const void*, void*, cudaStream_t); \
+  template cudaError_t launch_bc_flux<P>(const DGrid&, const SetArgs&, const BcMask&, const FluxPtrs&, int*,        \
+                                         cudaStream_t);                                                           \
   template cudaError_t launch_inittraj<P>(const DGrid&, float*, double*, cudaStream_t);                            \
   template cudaError_t launch_traject<P>(const DGrid&, const TrajArgs&, cudaStream_t);                             \
   template cudaError_t launch_traject_box<P>(const DGrid&, const TrajArgs&, int, int, int, int, cudaStream_t);      \

@@ -234,10 +234,17 @@ struct ZlfPtrs {
 };
 template <typename T>
 cudaError_t launch_bc_zlf(const BcMask& m, int setup, const ZlfPtrs& f, cudaStream_t s);
-template <typename T>
-cudaError_t launch_bc_mask(const BcMask& m, const void* src, void* mo, void* mi, cudaStream_t s);
-template <typename T>
-cudaError_t launch_bc_zero(const BcMask& m, void* fo, void* fi, cudaStream_t s);
+// tracers of one boundary-flux launch: src[q] NULL for the masks themselves
+struct FluxPtrs {
+  const void* src[kMaxFields];
+  void* fo[kMaxFields];
+  void* fi[kMaxFields];
+  int n;
+};
+// list: scratch of 1 + (points of range b) ints
+template <int PREC>
+cudaError_t launch_bc_flux(const DGrid& g, const SetArgs& a, const BcMask& m, const FluxPtrs& fp, int* list,
+                           cudaStream_t s);
 
 // bound of a dependency wait of the batch kernel: >= 1 s of 64 ns sleeps
 constexpr unsigned long long kDepSpins = 1ull << 24;
