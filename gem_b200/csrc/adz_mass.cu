@@ -7,7 +7,7 @@
 // Every mass is an FP64 sum of (field * air mass) * area mask over the core
 // region, the first product in the field type as the reference forms it.
 // Sums are deterministic: each block reduces a fixed slice in a fixed tree
-// order, then one thread per tracer adds the block partials in index order.
+// order, then one thread per sum adds the block partials in index order.
 // The order differs from the reference's sequential loop, so masses agree to
 // rounding (about 1e-15 relative), not bit for bit.
 #include <cuda_runtime.h>
@@ -245,15 +245,25 @@ __device__ __forceinline__ bool almost_zero(double a) {
 
 enum Stage { kAfterPMW = 0, kAfterFlux = 1, kAfterBcR = 2, kAfterBc = 3 };
 
-// one thread per tracer: partials in index order, then the scalar formulas
+// a block per tracer: the partials into shared memory, their sums in index
+// order by one thread per sum, then the scalar formulas.  One thread per
+// tracer reading them from memory took 60 to 167 us for 4 tracers, a third of
+// the pass it follows
 template <int STAGE>
-__global__ void k_finish(const double* __restrict__ part, State* __restrict__ st, int ntr,
-                         double* __restrict__ deficit, double* __restrict__ diag) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ntr) return;
-  double s[kSums] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = 0; b < kBlocks; b++)
-    for (int c = 0; c < kSums; c++) s[c] += part[((long long)q * kBlocks + b) * kSums + c];
+__global__ void __launch_bounds__(kThreads) k_finish(const double* __restrict__ part, State* __restrict__ st,
+                                                     double* __restrict__ deficit, double* __restrict__ diag) {
+  const int q = blockIdx.x;
+  __shared__ double sp[kBlocks * kSums], s[kSums];
+  for (int t = threadIdx.x; t < kBlocks * kSums; t += kThreads) sp[t] = part[(long long)q * kBlocks * kSums + t];
+  __syncthreads();
+  if (threadIdx.x < kSums) {
+    double v = 0.0;
+#pragma unroll 16
+    for (int b = 0; b < kBlocks; b++) v += sp[b * kSums + threadIdx.x];
+    s[threadIdx.x] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   State& S = st[q];
   if (STAGE == kAfterPMW) {
     S = State{};
@@ -461,7 +471,6 @@ int run_bc(int ntr, const adzc_bc_tracer* in, const void* airm_p, const void* ai
   const dim3 rg(kBlocks, ntr);
   const T* ap = (const T*)airm_p;
   const T* am = (const T*)airm_m;
-  const int fb = (ntr + 127) / 128;
   Geo gm = g;
   gm.mask = mask;
   // four passes over the fields: masses and weights; fluxes (boundary only);
@@ -470,18 +479,18 @@ int run_bc(int ntr, const adzc_bc_tracer* in, const void* airm_p, const void* ai
   const bool vb = vec_ok<T>(ntr, in, ap, am, mask, brange, gm);
   if (vc) k_reduce<T, kPMW, true><<<rg, kThreads, 0, s>>>(d_tr, core, gm, ap, am, d_part);
   else k_reduce<T, kPMW, false><<<rg, kThreads, 0, s>>>(d_tr, core, gm, ap, am, d_part);
-  k_finish<kAfterPMW><<<fb, 128, 0, s>>>(d_part, d_st, ntr, deficit, diag);
+  k_finish<kAfterPMW><<<ntr, kThreads, 0, s>>>(d_part, d_st, deficit, diag);
   if (vb) k_reduce<T, kFlux, true><<<rg, kThreads, 0, s>>>(d_tr, brange, gm, ap, am, d_part);
   else k_reduce<T, kFlux, false><<<rg, kThreads, 0, s>>>(d_tr, brange, gm, ap, am, d_part);
-  k_finish<kAfterFlux><<<fb, 128, 0, s>>>(d_part, d_st, ntr, deficit, diag);
+  k_finish<kAfterFlux><<<ntr, kThreads, 0, s>>>(d_part, d_st, deficit, diag);
   if (vc) k_correct<T, true><<<rg, kThreads, 0, s>>>(d_tr, d_st, core, gm, am, min_max, d_part);
   else k_correct<T, false><<<rg, kThreads, 0, s>>>(d_tr, d_st, core, gm, am, min_max, d_part);
   if (min_max) {
-    k_finish<kAfterBcR><<<fb, 128, 0, s>>>(d_part, d_st, ntr, deficit, diag);
+    k_finish<kAfterBcR><<<ntr, kThreads, 0, s>>>(d_part, d_st, deficit, diag);
     if (vc) k_scale<T, true><<<rg, kThreads, 0, s>>>(d_tr, d_st, core, gm, am, d_part);
     else k_scale<T, false><<<rg, kThreads, 0, s>>>(d_tr, d_st, core, gm, am, d_part);
   }
-  k_finish<kAfterBc><<<fb, 128, 0, s>>>(d_part, d_st, ntr, deficit, diag);
+  k_finish<kAfterBc><<<ntr, kThreads, 0, s>>>(d_part, d_st, deficit, diag);
   return cudaGetLastError() == cudaSuccess ? ADZC_OK : ADZC_ERR_CUDA;
 }
 
