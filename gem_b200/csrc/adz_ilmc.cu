@@ -37,7 +37,7 @@
 // lane's cells stay in registers, and the list entry and bounds of a warp's
 // next tile are loaded before the barrier.  Bounds and cubes of 3 tracers at
 // 301 x 262 x 80, 3.4 % of the points outside: 20.4 ms with a launch per
-// wavefront (15 us each), 9.2 ms here (6.7 us).
+// wavefront (15 us each), 8.8 ms here (6.5 us).
 // Built with -fmad=false: the REAL arithmetic is the reference's, without
 // contraction.
 #include <cuda_runtime.h>
@@ -279,7 +279,8 @@ __global__ void __launch_bounds__(1024) k_scan(const int* __restrict__ count, in
 }
 
 // every wavefront in turn: a warp per listed tile, its points in loop order,
-// then a barrier over the grid.  bar counts the blocks that have arrived.
+// then a barrier over the grid.  64 registers up to two FP32 sweeps (10.5 ms at
+// the 74 that ptxas takes, 9.6 at 64).  bar counts the blocks that have arrived.
 // The wait is bounded: when it runs out the block raises kErrTimeout and
 // leaves, and so do the others.
 template <typename T, int S>
@@ -403,7 +404,7 @@ namespace {
 
 using namespace adz::ilmc;
 
-// the cooperative launch of every wavefront, two blocks per SM
+// the cooperative launch of every wavefront, one block per SM
 template <typename T, int S>
 cudaError_t launch_waves(const Box& b, const Fields<T>& fl, const T* air, int nwave, int c1, int ntile,
                          const int* wstart, const int* list, unsigned long long* bar, int* status, cudaStream_t s) {
@@ -415,7 +416,7 @@ cudaError_t launch_waves(const Box& b, const Fields<T>& fl, const T* air, int nw
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_waves<T, S>, 32 * kWarps, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-  const int grid = sms * std::min(per_sm, 2);
+  const int grid = sms;  // two per SM lengthen the barrier: 9.9 against 9.6 ms (8 tracers at 1024 x 1024 x 80: 77.9, 77.0)
   Box bb = b;
   Fields<T> ff = fl;
   void* args[] = {&bb, &ff, &air, &nwave, &c1, &ntile, &wstart, &list, &bar, &status};
