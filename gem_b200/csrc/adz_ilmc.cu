@@ -174,6 +174,7 @@ __device__ __forceinline__ void visit_warp(const Box& b, const Cells<S>& cl, T* 
   const T aire = __ldg(air + e);
 #pragma unroll
   for (int sw = 1; sw <= S; sw++) {
+    if ((over ? o_shoot : u_shoot) == (T)0) break;  // nothing left to move: the later sweeps change nothing
     const int q0 = first_slot(sw), nq = shell_len(sw);
     T cap[shell_slots(S)];
 #pragma unroll
