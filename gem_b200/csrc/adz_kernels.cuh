@@ -1507,9 +1507,8 @@ cudaError_t launch_inittraj(const DGrid& g, float* pxyzm, double* wpxyz, cudaStr
 
 template <int PREC>
 cudaError_t launch_traject(const DGrid& g, const TrajArgs& a, cudaStream_t s) {
-  if constexpr (PREC != kRef32)
-    if (st_grid_ok<PREC>(g, a.k00, g.nj))
-      return st_launch_traject<PREC, false>(g, a, 1, g.ni, 1, g.nj, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
+  if (st_grid_ok<PREC>(g, a.k00, g.nj))
+    return st_launch_traject<PREC, false>(g, a, 1, g.ni, 1, g.nj, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
 #if ADZ_TRAJ_TILE_K > 1
   constexpr int TK = ADZ_TRAJ_TILE_K, TI = ADZ_TRAJ_TILE_I;
   const long long nb = (long long)((g.ni + TI - 1) / TI) * ((g.nk - a.k00 + 1 + TK - 1) / TK) * g.nj;
@@ -1527,9 +1526,8 @@ cudaError_t launch_traject_box(const DGrid& g, const TrajArgs& a, int i0, int nx
   const long long nkp = g.nk - a.k00 + 1, n = (long long)nx * ny * nkp;
   if (n <= 0) return cudaSuccess;
   if (batch_use_tiles(nx, nkp)) {
-    if constexpr (PREC != kRef32)
-      if (st_grid_ok<PREC>(g, a.k00, ny))
-        return st_launch_traject<PREC, false>(g, a, i0, nx, j0, ny, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
+    if (st_grid_ok<PREC>(g, a.k00, ny))
+      return st_launch_traject<PREC, false>(g, a, i0, nx, j0, ny, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
     const long long nb = (long long)((nx + 31) / 32) * ((nkp + 3) / 4) * ny;
     if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;
     k_traject_box<PREC, true><<<(unsigned)nb, 128, 0, s>>>(g, a, i0, nx, j0, ny);

@@ -37,14 +37,16 @@ struct StShape {
 // iteration to a tolerance takes 3 blocks (80 registers): the first step of a
 // run at 768 x 640 x 80 8.77 ms, 9.07 at 4 blocks, 9.65 with the direct kernel.
 // FP64: one box of interleaved (u, v, w) cells; 1024 x 512 x 80 6.01 ms,
-// direct 8.43 (2 x 4 points at 2 blocks 6.20).  REF32 stays direct: its
-// conversions to FP64 bound it either way
+// direct 8.43 (2 x 4 points at 2 blocks 6.20); REF32, the same box of FP32
+// cells at 4 blocks (80 registers), 5.81, direct 6.25
 template <int PREC>
 struct TrajBox;
 template <>
 struct TrajBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
 template <>
 struct TrajBox<kFp64> : StShape<3, 2, 3, 48, 8, 8> {};
+template <>
+struct TrajBox<kRef32> : StShape<3, 2, 4, 64, 8, 8> {};
 template <int PREC>
 struct SetBox;
 // 8 fields of set t at 1024 x 1024 x 80: 7.93 ms, direct 11.19 (rows that are
@@ -59,8 +61,8 @@ constexpr int kStRing = 3;  // boxes in flight of the sets kernel
 // fields from which a part of a sets launch is staged: placing and filling
 // the boxes costs about what two fields gain (MIXED at 1024 x 1024 x 80, 2
 // fields: 3.44 ms staged, 3.36 direct; 5 fields 5.64 and 7.19; FP64 at 1024 x
-// 512 x 80, 2 fields: 3.14 and 2.85, 5 fields 5.07 and 5.95).  REF32 stays
-// direct: its conversions bound it (8 fields: 6.93 staged, 6.38 direct)
+// 512 x 80, 2 fields: 3.14 and 2.85, 5 fields 5.07 and 5.95).  The sets of
+// REF32 stay direct (8 fields: 6.88 staged, 6.37 direct)
 constexpr int kStMinFields = 3, kStQvMinFields = 2;
 
 // a staged box: first cell in the extended array, extents in cells
@@ -452,11 +454,13 @@ __device__ __forceinline__ void st_winds(const DGrid& g, const typename Types<PR
   } else {
     double cf[20];
     int off;
-    coef_f64pos(cf, off, px, py, pz, g.tab_m);
+    if constexpr (PREC == kRef32) coef_f32pos(cf, off, (float)px, (float)py, (float)pz, g.tab_m);
+    else coef_f64pos(cf, off, px, py, pz, g.tab_m);
     const F* s = sm + 3 * o;
-    ud = st_interp3_exact<F, RP, PP>(s, d0, d3, cf);
-    vd = st_interp3_exact<F, RP, PP>(s + 1, d0, d3, cf);
-    wd = st_interp3_exact<F, RP, PP>(s + 2, d0, d3, cf);
+    // Tricublin_zyx3_n returns ``real`` (F)
+    ud = (double)(F)st_interp3_exact<F, RP, PP>(s, d0, d3, cf);
+    vd = (double)(F)st_interp3_exact<F, RP, PP>(s + 1, d0, d3, cf);
+    wd = (double)(F)st_interp3_exact<F, RP, PP>(s + 2, d0, d3, cf);
   }
 }
 
