@@ -542,9 +542,9 @@ def workload_config(args, ws, decomp=None):
             "points_per_step": ni * nj * nk, "l2": "inputs larger than L2 (no flush)", "parallelism": par}
 
 
-# kernels of one MIXED step: departure winds, trajectory, and one
-# interpolation launch per position set (u, v, then w + tracers at thermo points)
-LAUNCHES_PER_STEP = 3  # k_prepare, k_traject, k_tricub_parts (every set's field groups)
+# kernels of one MIXED step: departure winds, trajectory, w with the tracers
+# from shared-memory boxes, and u and v in one direct launch
+LAUNCHES_PER_STEP = 4  # k_prepare4, k_traject_st, k_sets_st (three or more fields), k_tricub_parts
 HALO_LAUNCHES_PER_STEP = 4  # pack + unpack of the two exchanges (N > 1)
 
 
@@ -719,8 +719,9 @@ def measure_batch(args, timed, ws, cfgs, label):
             ad.adz_traject(prec, cfg.dt, inp, None, wp)
             ad.adz_tricub_sets(prec, [0, 1, 1, len(srcs) - 2], srcs, dsts, mono)
     ms_s, _ = timed(sequential, args.steps, args.warmup)
-    # per domain: winds, trajectory, and every set's field groups in one launch
-    seq_launches = 3 * len(doms)
+    # per domain: winds, trajectory, u and v, and w with the tracers (a launch of
+    # its own from three fields on)
+    seq_launches = sum(3 + (1 + c.ntracers >= 3) for c in cfgs)
     plan = batch.query()
     nl = {"one launch": 1, "phased (one launch per phase)": 3}.get(plan["plan"], seq_launches)
     out = {"workload": f"{len(cfgs)} {label}",

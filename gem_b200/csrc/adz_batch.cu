@@ -24,7 +24,7 @@
 // graph, one per phase, each kernel with the register budget of the
 // per-domain kernel of its phase; launch order replaces the dependency waits.
 // The per-domain plan replays every domain's own launches in turn: departure
-// winds, trajectory and all field groups in one k_tricub_parts launch, as the
+// winds, trajectory and the field groups (launch_tricub_parts), as the
 // per-domain entry points run them.  The tuner weighs the phased and
 // per-domain plans against the one-launch kernel's budgets.
 #include <cuda_runtime.h>
@@ -131,8 +131,7 @@ int build_items(adzc_batch* b, int rows) {
   return ADZC_OK;
 }
 
-// one domain's own launches: departure winds, trajectory and all field
-// groups in one k_tricub_parts launch
+// one domain's own launches: departure winds, trajectory and the field groups
 template <int PREC>
 cudaError_t enqueue_domain(const adz::BDom& D, cudaStream_t s) {
   cudaError_t e = adz::launch_prepare<PREC>(D.g, D.uu, D.vv, D.ww, const_cast<void*>(D.ta.uvw_d), s);

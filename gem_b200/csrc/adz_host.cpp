@@ -1072,7 +1072,7 @@ extern "C" int adzc_tricub_sets(adzc_handle* h, int prec, const int* nfields, co
     if (!srcs[f] || !dsts[f] || !mono_ok(mono ? mono[f] : 0, set)) return fail(ADZC_ERR_ARG);
   }
   // every tricubic field group of every set in one interleaved launch
-  // (k_tricub_parts); BICUBH_QV fields of set t after it
+  // (launch_tricub_parts); BICUBH_QV fields of set t after it
   const adz::SetArgs a = set_args(h);
   const cudaStream_t s = (cudaStream_t)stream;
   adz::SetParts sp{};

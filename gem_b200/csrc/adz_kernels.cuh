@@ -8,6 +8,10 @@
 //   k_tricub_set   position of a set derived in registers (B/adz_interp_traj.F90)
 //                  then the multi-field interpolation, mono bounds and clip
 //                  (B/adz_interp_hlt.F90:98-182, B/adz_post_tr.F90:81-94)
+//   k_traject_st, k_sets_st, k_qv_st  the same on shared-memory boxes, where
+//                  that is faster (adz_staged.cuh); the kernels above gather
+//                  straight from memory
+//   k_bc_flux, k_bc_edge  LAM boundary fluxes (B/adz_BC_LAM_Aranami_hlt.F90)
 //   k_interp_pos   the reference interpolators on explicit positions
 //                  (B/turbo_tricublin.c:752-1312)
 // B/ = src/gemdyn/src/base/.
@@ -1551,11 +1555,12 @@ cudaError_t launch_prepare_box(const DGrid& g, const void* uu, const void* vv, c
 template <int PREC>
 cudaError_t launch_traject_tol(const DGrid& g, const TrajArgs& a, double tol, int maxit, unsigned char* iters,
                                unsigned long long* stats, cudaStream_t s, const GuessStart& gs) {
-#ifndef ADZ_NO_ST_TOL
+  // FP64 stays direct (not measured staged).  Rows that are no multiple of 16
+  // bytes gain less (first step of a run at 765 x 640 x 80: 10.33 ms staged, 10.62
+  // direct; 768: 8.76 and 9.65)
   if constexpr (PREC == kMixed)
     if (st_grid_ok<PREC>(g, a.k00, g.nj))
       return st_launch_traject<PREC, true>(g, a, 1, g.ni, 1, g.nj, tol, maxit, iters, stats, gs, s);
-#endif
 #if ADZ_TOL_TILES
   const long long nb = (long long)((g.ni + 31) / 32) * ((g.nk - a.k00 + 1 + 3) / 4) * g.nj;
   if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;

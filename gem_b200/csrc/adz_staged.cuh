@@ -145,6 +145,13 @@ __device__ __forceinline__ StBox st_box(const DGrid& g, const int* red, int al) 
   return b;
 }
 
+// the reduced stencils span more than a box of shape C (uniform over the block)
+template <class C>
+__device__ __forceinline__ bool st_overflow(const int* red, int al) {
+  return red[0] != 0x7fffffff && (4 - red[3] - (red[0] & ~(al - 1)) > C::RP || 4 - red[4] - red[1] > C::BY ||
+                                  1 - red[5] - red[2] > C::BZ);
+}
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -470,7 +477,8 @@ __device__ __forceinline__ void st_winds(const DGrid& g, const typename Types<PR
 // points move by their whole displacement, so there the box is placed again
 // when more than 1/16 of the block's points left it.
 // TOL: the iteration to a tolerance (traject_point_tol), MIXED; its start is
-// smooth and the first update scatters the levels, so its box has a margin.
+// smooth and the first update scatters the levels, so its box has a margin
+// (a margin of levels only: 8.98 against 8.76 ms).
 // Else a.niter updates.
 template <int PREC, bool TOL>
 __global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MINB)
@@ -509,6 +517,15 @@ __global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MI
     st_reduce(red, use, c);
     __syncthreads();
     box = st_box<C, TOL>(g, red, vec ? AL : 1);
+    // FP64, REF32: where more than a quarter of the points would be left out
+    // (strong shear inside the tile), the direct code takes them all (83 x 192 x
+    // 59 at Courant numbers up to 2: 0.217 against 0.25 ms).  In the MIXED
+    // kernel the test costs more in spills (7.8 against 6.9 ms) than it saves
+    if constexpr (PREC != kMixed)
+      if (st_overflow<C>(red, vec ? AL : 1) && __syncthreads_count(use && !st_in_box(box, c)) > C::NT / 4) {
+        box.nx = 0;
+        return;
+      }
     const F* uvw = (const F*)a.uvw_d;
     if constexpr (PREC == kMixed) {
       StCopy<F, C> cp;
@@ -803,6 +820,11 @@ __global__ void __launch_bounds__(QvBox::NT, QvBox::MINB)
   st_reduce(red, in, cell);
   __syncthreads();
   const StBox box = st_box<C, false>(g, red, vec ? 4 : 1);
+  // more than a quarter of the points outside the box: the direct code for all
+  if (st_overflow<C>(red, vec ? 4 : 1) && __syncthreads_count(in && !st_in_box(box, cell)) > C::NT / 4) {
+    if (active) qv_point_direct<PREC>(&g, &a, &fp, i, j, k);
+    return;
+  }
   StCopy<float, C> cp;
   cp.plan(box, g, vec != 0);
   auto copy = [&](int q, int slot) {

@@ -483,8 +483,10 @@ int adzc_bermejo_conde(adzc_handle *h, int prec, int ntr, const adzc_bc_tracer *
  * when min_max (adz_ILMC_min_max_L).  Bit-exact with the reference's
  * sequential loop order, run as wavefronts of row tiles whose neighbourhoods
  * never interact, all tracers (at most ADZC_ILMC_MAX_TRACERS) together;
- * rounds (may be NULL) receives the number of wavefronts.  Does not
- * synchronise the stream. */
+ * rounds (may be NULL) receives the number of wavefronts.  One cooperative
+ * launch runs the wavefronts, with a bounded wait between them
+ * (ADZC_ERR_TIMEOUT in adzc_status when it runs out).  Does not synchronise
+ * the stream. */
 #define ADZC_ILMC_MAX_TRACERS 32
 int adzc_ilmc(adzc_handle *h, int prec, int ntr, void *const *f, const void *const *mn, const void *const *mx,
               const void *air, int sweep_max, int min_max, int *rounds, void *stream);
