@@ -37,7 +37,7 @@
 // lane's cells stay in registers, and the list entry and bounds of a warp's
 // next tile are loaded before the barrier.  Bounds and cubes of 3 tracers at
 // 301 x 262 x 80, 3.4 % of the points outside: 20.4 ms with a launch per
-// wavefront (15 us each), 8.8 ms here (6.5 us).
+// wavefront (15 us each), 8.1 ms here (6 us).
 // Built with -fmad=false: the REAL arithmetic is the reference's, without
 // contraction.
 #include <cuda_runtime.h>
