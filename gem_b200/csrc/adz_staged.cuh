@@ -86,15 +86,17 @@ __device__ __forceinline__ StCell st_cell(const DGrid& g, const DZtab& lv, doubl
   cell_of(pz, iz);
   iz = imin_(imax_(iz, 1), lv.nk - 1);
   StCell c;
-  c.ci = ix + lv.offi - 1 - g.lminx;
-  c.cj = iy + lv.offj - 1 - g.lminy;
+  c.ci = (int)((unsigned)ix + (unsigned)(lv.offi - 1 - g.lminx));  // a cell at the end of the range of int wraps
+  c.cj = (int)((unsigned)iy + (unsigned)(lv.offj - 1 - g.lminy));
   c.iz0 = iz - 1;
   c.zl = c.iz0 < 1 || c.iz0 > lv.nk - 3;
   return c;
 }
-// the 4 x 4 columns lie in the extended array (planes always do)
+// the 4 x 4 columns lie in the extended array (planes always do; nit and njt
+// are 5 or more).  Unsigned: c.ci + 3 would wrap for the last three ints, the
+// cells of REF32's stored positions (not clipped) beyond the range of int
 __device__ __forceinline__ bool st_inside(const DGrid& g, const StCell& c) {
-  return c.ci >= 0 && c.ci + 3 < g.nit && c.cj >= 0 && c.cj + 3 < g.njt;
+  return (unsigned)c.ci < (unsigned)(g.nit - 3) && (unsigned)c.cj < (unsigned)(g.njt - 3);
 }
 // the stencil lies in the box
 template <class Cell>

@@ -126,3 +126,37 @@ def test_boundary_flux_shared_and_many():
     assert ad.status() == 0 and float(fi[0].abs().max()) > 0 and float(fo[0].abs().max()) > 0
     for q in range(len(srcs)):
         assert torch.equal(fo[q][m], go[q][m]) and torch.equal(fi[q][m], gi[q][m])
+
+
+# REF32 starts from the stored FP32 positions as they are.  maxcfl 1 (halo 2):
+# the stencil corner of a position beyond the range of int is its last int.
+# Not a number counts as cell 0, and the winds found there as not finite
+@pytest.mark.parametrize("bad,status", [(float("nan"), 5), (3e9, 4), (-3e9, 4), (float("inf"), 4), (-float("inf"), 4)])
+def test_ref32_position_without_a_cell(bad, status):
+    """A point whose stored position has no cell in the array is reported as
+    such and left as it is; the others are untouched by it."""
+    from gem_b200 import adz as A, synth
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    cfg = synth.config_small(70, 21, 9)
+    cfg.maxcfl, cfg.dt = 1, 60.0
+    inp = synth.make_inputs(cfg, device="cuda", dtype=torch.float32)
+    ad = A.Adz.from_config(cfg, lam=False)
+    px, wp = ad.new_state(A.REF32)
+    ad.adz_inittraj(A.REF32, px, wp)
+    ad.adz_traject(A.REF32, cfg.dt, inp, px, wp)
+    start_px, start_wp = px.clone(), wp.clone()
+    ad.adz_traject(A.REF32, cfg.dt, inp, px, wp)
+    torch.cuda.synchronize()
+    assert ad.status() == 0
+    for k, j, i in ((0, 0, 0), (4, 10, 2), (8, 20, 69)):
+        px2, wp2 = start_px.clone(), start_wp.clone()
+        px2[k, j, i, 0] = bad
+        before = px2[k, j, i].clone()
+        ad.adz_traject(A.REF32, cfg.dt, inp, px2, wp2)
+        torch.cuda.synchronize()
+        assert ad.status() == status
+        assert torch.equal(_bits(px2[k, j, i]), _bits(before))
+        px2[k, j, i] = px[k, j, i]
+        wp2[:, k, j + 2, i + 2] = wp[:, k, j + 2, i + 2]
+        assert torch.equal(_bits(px2), _bits(px)) and torch.equal(_bits(wp2), _bits(wp))
