@@ -891,6 +891,30 @@ extern "C" int adzc_interp_traj(adzc_handle* h, int prec, int set, void* pos, vo
   return ADZC_OK;
 }
 
+constexpr int kFluxGroup = adz::kMaxFields / 2;  // tracers of a boundary-flux launch (two fluxes each)
+
+extern "C" int adz_internal_flux_copies(int ntr, const void* const* srcs, void* const* fo, void* const* fi, size_t ext,
+                                        unsigned char* when) {
+  auto shares = [&](const void* p, int r0, int r1) {
+    for (int r = r0; r < r1; r++)
+      for (const void* o : {(const void*)fo[r], (const void*)fi[r]})
+        if ((const char*)p < (const char*)o + ext && (const char*)o < (const char*)p + ext) return true;
+    return false;
+  };
+  int before = 0, most = 0;
+  for (int q0 = 0; q0 < ntr; q0 += kFluxGroup) {
+    const int q1 = std::min(q0 + kFluxGroup, ntr);
+    int own = 0;
+    for (int q = q0; q < q1; q++) {
+      when[q] = !srcs[q] ? 0 : shares(srcs[q], 0, q0) ? 2 : shares(srcs[q], q0, q1) ? 1 : 0;
+      before += when[q] == 2;
+      own += when[q] == 1;
+    }
+    most = std::max(most, own);
+  }
+  return before + most;
+}
+
 extern "C" int adzc_bc_lam_flux(adzc_handle* h, int prec, int ntr, const void* const* srcs, void* const* fo,
                                 void* const* fi, void* stream) {
   AdzRange nvtx_range("adz_BC_LAM_Aranami_hlt");
@@ -910,35 +934,37 @@ extern "C" int adzc_bc_lam_flux(adzc_handle* h, int prec, int ntr, const void* c
   adz::SetArgs a = set_args(h);
   a.pert = nullptr;  // the fluxes are plain interpolations (tricublin_zyx1_m_n)
   const cudaStream_t s = (cudaStream_t)stream;
-  for (int q0 = 0; q0 < ntr; q0 += adz::kMaxFields / 2) {
+  // tracers that share memory with the flux arrays are read from copies.  The
+  // scratch of every group is taken before the first launch: growing it frees
+  // what queued launches read, and fails under capture
+  const size_t ext = (size_t)D.nij * D.nk * field_bytes(prec);
+  const size_t nlist = 1 + (size_t)nxb * nyb * D.nk;
+  std::vector<unsigned char> when(ntr);
+  const size_t ncopy = (size_t)adz_internal_flux_copies(ntr, srcs, fo, fi, ext, when.data());
+  void* scratch = nullptr;
+  if (adz_internal_aux(h, ncopy * ext + nlist * sizeof(int), &scratch) != ADZC_OK) return fail(ADZC_ERR_ALLOC);
+  int* list = (int*)((char*)scratch + ncopy * ext);
+  std::vector<const void*> from(srcs, srcs + ntr);
+  char* c = (char*)scratch;
+  auto copy = [&](int q) {
+    const cudaError_t e = cudaMemcpyAsync(c, srcs[q], ext, cudaMemcpyDeviceToDevice, s);
+    from[q] = c;
+    c += ext;
+    return e;
+  };
+  for (int q = 0; q < ntr; q++)
+    if (when[q] == 2) ADZ_CK(copy(q));
+  char* const own = c;  // the copies of a group's own tracers, one group after another
+  for (int q0 = 0; q0 < ntr; q0 += kFluxGroup) {
     adz::FluxPtrs fp{};
-    fp.n = std::min(adz::kMaxFields / 2, ntr - q0);
+    fp.n = std::min(kFluxGroup, ntr - q0);
+    c = own;
     for (int q = 0; q < fp.n; q++) {
-      fp.src[q] = srcs[q0 + q];
+      if (when[q0 + q] == 1) ADZ_CK(copy(q0 + q));
+      fp.src[q] = from[q0 + q];
       fp.fo[q] = fo[q0 + q];
       fp.fi[q] = fi[q0 + q];
     }
-    // a tracer that shares memory with a flux array of its group is read from a copy
-    const size_t ext = (size_t)D.nij * D.nk * field_bytes(prec);
-    auto shares = [&](const void* p) {
-      for (int r = 0; p && r < fp.n; r++)
-        for (const void* o : {(const void*)fp.fo[r], (const void*)fp.fi[r]})
-          if ((const char*)p < (const char*)o + ext && (const char*)o < (const char*)p + ext) return true;
-      return false;
-    };
-    size_t ncopy = 0;
-    for (int q = 0; q < fp.n; q++) ncopy += shares(fp.src[q]);
-    const size_t nlist = 1 + (size_t)nxb * nyb * D.nk;
-    void* scratch = nullptr;
-    if (adz_internal_aux(h, ncopy * ext + nlist * sizeof(int), &scratch) != ADZC_OK) return fail(ADZC_ERR_ALLOC);
-    char* c = (char*)scratch;
-    for (int q = 0; ncopy > 0 && q < fp.n; q++)
-      if (shares(fp.src[q])) {
-        ADZ_CK(cudaMemcpyAsync(c, fp.src[q], ext, cudaMemcpyDeviceToDevice, s));
-        fp.src[q] = c;
-        c += ext;
-      }
-    int* list = (int*)c;
     switch (prec) {
       case ADZC_REF32: ADZ_CK(adz::launch_bc_flux<adz::kRef32>(D, a, m, fp, list, s)); break;
       case ADZC_FP64: ADZ_CK(adz::launch_bc_flux<adz::kFp64>(D, a, m, fp, list, s)); break;

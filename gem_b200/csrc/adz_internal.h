@@ -25,6 +25,13 @@ int adz_internal_fail(int status);
 int adz_internal_scratch(adzc_handle* h, int prec, void** uvw, void** wdep);
 // a handle-owned device buffer of at least bytes for auxiliary passes (mass fixers)
 int adz_internal_aux(adzc_handle* h, size_t bytes, void** p);
+// the tracers of a boundary-flux call that are read from copies because they
+// share memory with flux arrays (ext bytes each): when[q] 1 with an array of
+// the tracer's own group (copied before that group), 2 with one that an earlier
+// group writes (copied before the first), 0 none; returns the copies that
+// exist at a time
+extern "C" int adz_internal_flux_copies(int ntr, const void* const* srcs, void* const* fo, void* const* fi, size_t ext,
+                                        unsigned char* when);
 // the optional inputs of the position sets registered on the handle: the
 // surface-layer winds (adzc_slt_winds) and the perturbation pattern
 // (adzc_rhs_perturbation); NULL when not set

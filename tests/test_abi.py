@@ -66,6 +66,38 @@ def test_errors_without_device(L):
     assert L.adzc_ztab_create(lev.ctypes.data, 3, 10, 10, 0, 0, C.byref(out)) == 3  # nk < 4
 
 
+def test_boundary_flux_copies(L):
+    """Which tracers of a boundary-flux call are read from copies, and how many
+    copies exist at a time (groups of 8 tracers)."""
+    ext = 4096
+
+    def plan(srcs, fo, fi):
+        n = len(srcs)
+        arr = lambda v: (C.c_void_p * n)(*v)  # noqa: E731
+        when = (C.c_ubyte * n)()
+        f = L.adz_internal_flux_copies
+        f.argtypes = [C.c_int] + [C.c_void_p] * 3 + [C.c_size_t, C.c_void_p]
+        return f(n, arr(srcs), arr(fo), arr(fi), ext, when), list(when)
+
+    at = lambda q: 0x10000 + q * ext  # noqa: E731
+    n = 19
+    src, fo, fi = ([at(100 * b + q) for q in range(n)] for b in range(3))
+    assert plan(src, fo, fi) == (0, [0] * n)
+    # a tracer in its own flux array, one that overlaps it by a byte, one that only touches it
+    s = list(src)
+    s[1], s[2], s[3] = fo[1], fi[2] + ext - 1, fo[n - 1] + ext
+    assert plan(s, fo, fi) == (2, [0, 1, 1] + [0] * 16)
+    # the largest group decides: one copy in the first, three in the second
+    s = list(src)
+    s[0], s[8], s[9], s[15] = fo[0], fo[9], fi[8], fo[15]
+    assert plan(s, fo, fi) == (3, [1] + [0] * 7 + [1, 1] + [0] * 5 + [1] + [0] * 3)
+    # an array of an earlier group; an array of a later group is written after the tracer was read
+    s = list(src)
+    s[17], s[18], s[3], s[4] = fi[0], fo[16], fo[18], None
+    got = plan(s, fo, fi)
+    assert got[0] == 2 and [got[1][q] for q in (3, 4, 17, 18)] == [0, 0, 2, 1]
+
+
 def test_no_library_no_fallback(monkeypatch, tmp_path):
     """Without the built library every entry point raises: there is no CPU
     fallback behind the binding."""

@@ -106,7 +106,8 @@ def test_staged_sets_equal_direct(prec_name, qv, n, size, wild, offset):
 
 
 def test_boundary_flux_shared_and_many():
-    """More tracers than one launch takes, one of them in its own flux array."""
+    """More tracers than one launch takes; one of them in its own flux array,
+    two more in the flux arrays of the tracers before them."""
     A, cfg, prec, ft, inp = _case("mixed", (56, 44, 12), False, 11)
     ad = A.Adz.from_config(cfg)
     _, wp = ad.new_state(prec)
@@ -120,6 +121,8 @@ def test_boundary_flux_shared_and_many():
     own = inp["tracers"][2].clone()
     srcs = list(inp["tracers"])
     srcs[2] = go[2] = own
+    srcs[9] = go[0] = inp["tracers"][9].clone()
+    srcs[10] = gi[8] = inp["tracers"][10].clone()
     m = ad.range_mask(A.SET_B, device="cuda")
     ad.bc_lam_flux(prec, srcs, go, gi)
     torch.cuda.synchronize()
