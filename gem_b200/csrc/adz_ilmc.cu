@@ -40,6 +40,7 @@
 // wavefront (15 us each), 8.1 ms here (6 us).
 // Built with -fmad=false: the REAL arithmetic is the reference's, without
 // contraction.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -405,7 +406,35 @@ namespace {
 
 using namespace adz::ilmc;
 
-// the cooperative launch of every wavefront, one block per SM
+// SMs that the kernels of a stream run on: all of the device's, or those of
+// the green context that the stream belongs to
+int stream_sms(cudaStream_t s, int sms) {
+  struct Driver {
+    CUresult (*stream_ctx)(CUstream, CUcontext*, CUgreenCtx*) = nullptr;
+    CUresult (*resource)(CUgreenCtx, CUdevResource*, CUdevResourceType) = nullptr;
+    Driver() {  // through the runtime: the library loads without a driver
+      cudaDriverEntryPointQueryResult q;
+      void* p = nullptr;
+      if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &p, 12050, cudaEnableDefault, &q) != cudaSuccess || !p)
+        return;
+      stream_ctx = (decltype(stream_ctx))p;
+      p = nullptr;
+      if (cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &p, 12040, cudaEnableDefault, &q) == cudaSuccess)
+        resource = (decltype(resource))p;
+    }
+  };
+  static const Driver d;
+  CUcontext ctx = nullptr;
+  CUgreenCtx green = nullptr;
+  CUdevResource r{};
+  if (!d.stream_ctx || !d.resource || d.stream_ctx((CUstream)s, &ctx, &green) != CUDA_SUCCESS || !green ||
+      d.resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS || r.sm.smCount < 1)
+    return sms;
+  return std::min(sms, (int)r.sm.smCount);
+}
+
+// the cooperative launch of every wavefront, one block per SM of the stream
+// (all of them run at once; a tile loop strides by the grid, so any number does)
 template <typename T, int S>
 cudaError_t launch_waves(const Box& b, const Fields<T>& fl, const T* air, int nwave, int c1, int ntile,
                          const int* wstart, const int* list, unsigned long long* bar, int* status, cudaStream_t s) {
@@ -417,7 +446,7 @@ cudaError_t launch_waves(const Box& b, const Fields<T>& fl, const T* air, int nw
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_waves<T, S>, 32 * kWarps, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-  const int grid = sms;  // two per SM lengthen the barrier: 9.9 against 9.6 ms (8 tracers at 1024 x 1024 x 80: 77.9, 77.0)
+  const int grid = stream_sms(s, sms);  // two per SM lengthen the barrier: 9.9 against 9.6 ms (8 tracers at 1024 x 1024 x 80: 77.9, 77.0)
   Box bb = b;
   Fields<T> ff = fl;
   void* args[] = {&bb, &ff, &air, &nwave, &c1, &ntile, &wstart, &list, &bar, &status};

@@ -86,3 +86,32 @@ def test_ilmc_wavefront_sizes(prec_name, size, ntr, frac, sweeps):
         ref = st.ilmc(t[0], t[1], t[2], air, sweep_max=sweeps, min_max=False)
         assert np.array_equal(g.cpu().numpy(), ref)
         assert not np.array_equal(ref, t[0])
+
+
+@pytest.mark.parametrize("prec_name,sweeps", [("ref32", 2), ("fp64", 3)])
+def test_ilmc_on_part_of_the_sms(prec_name, sweeps):
+    """A stream of a green context owns some of the SMs: the filter's blocks,
+    which run at once, must fit there."""
+    from gem_b200 import adz as A, synth
+    from oracle import oracle as O
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    prec = A.PREC_NAMES[prec_name]
+    cfg = synth.config_small(40, 36, 12)
+    st = O.Step(cfg, "oracle", "f64" if prec == A.FP64 else "f32")
+    dt = np.float64 if prec == A.FP64 else np.float32
+    t = _fields(st, dt, 0.05, 21)
+    ad = A.Adz.from_config(cfg)
+    f, mn, mx, air = (torch.from_numpy(x.copy()).cuda() for x in t)
+    torch.cuda.synchronize()
+    part = torch.cuda.GreenContext.create(num_sms=16, device_id=0)
+    part.set_context()
+    try:
+        A.ilmc(ad, prec, [f], [mn], [mx], air, sweep_max=sweeps, min_max=False)
+        torch.cuda.current_stream().synchronize()
+    finally:
+        part.pop_context()
+    torch.cuda.synchronize()
+    assert ad.status() == 0
+    ref = st.ilmc(t[0], t[1], t[2], air=t[3], sweep_max=sweeps, min_max=False)
+    assert np.array_equal(f.cpu().numpy(), ref) and not np.array_equal(ref, t[0])
