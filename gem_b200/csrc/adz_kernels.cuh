@@ -107,18 +107,15 @@
 #define ADZ_QV_BOUNDS __launch_bounds__(128)
 #endif
 
-// MIXED stores the departure winds as three component planes (u, v, w) instead
-// of interleaved triplets: each component gather is then a run of consecutive
-// floats across the warp's lanes, like a single field.
-#ifndef ADZ_MIXED_SOA
-#define ADZ_MIXED_SOA 1
-#endif
-
 namespace adz {
 
+// MIXED stores the departure winds as three component planes (u, v, w) instead
+// of interleaved triplets: each component gather is then a run of consecutive
+// floats across the warp's lanes, like a single field.  The boxes of
+// k_traject_st<kMixed> are copied from planes.
 template <int PREC>
 struct WindLayout {
-  static constexpr bool soa = (PREC == kMixed) && (ADZ_MIXED_SOA != 0);
+  static constexpr bool soa = PREC == kMixed;
 };
 
 // offsets into the extended, the (ni,nj,nk) and the Adz_wpxyz arrays; the
@@ -385,17 +382,11 @@ __device__ __forceinline__ int traj_update(const DGrid& g, const TrajArgs& a, in
     coef_mixed(w, px, py, pz, g.tab_m);
     off = w.off;
     if (!stencil_ok(g, off)) return kErrHalo;
-    if (WindLayout<PREC>::soa) {
-      const long long ncell = g.nij * g.nk;
-      const float* fu = (const float*)uvw + e111 + off;
-      ud = interp1_mixed<COH>(fu, w, g.tab_m.ni, g.tab_m.nij);
-      vd = interp1_mixed<COH>(fu + ncell, w, g.tab_m.ni, g.tab_m.nij);
-      wd = interp1_mixed<COH>(fu + 2 * ncell, w, g.tab_m.ni, g.tab_m.nij);
-    } else {
-      float o[3];
-      interp3_mixed<COH>((const float*)f3 + 3LL * off, w, g.tab_m.ni, g.tab_m.nij, o);
-      ud = o[0]; vd = o[1]; wd = o[2];
-    }
+    const long long ncell = g.nij * g.nk;
+    const float* fu = (const float*)uvw + e111 + off;
+    ud = interp1_mixed<COH>(fu, w, g.tab_m.ni, g.tab_m.nij);
+    vd = interp1_mixed<COH>(fu + ncell, w, g.tab_m.ni, g.tab_m.nij);
+    wd = interp1_mixed<COH>(fu + 2 * ncell, w, g.tab_m.ni, g.tab_m.nij);
   } else {
     double c[20];
     int zl;

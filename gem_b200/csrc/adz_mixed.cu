@@ -1,6 +1,6 @@
 // MIXED instantiation: FP64 positions and cell offsets, FP32 weights and
 // packed FP32 sums.  Departure winds are stored as three component planes
-// (ADZ_MIXED_SOA in adz_kernels.cuh).  Block shapes and resident blocks per
+// (WindLayout in adz_kernels.cuh).  Block shapes and resident blocks per
 // SM of the direct kernels (adz_staged.cuh has the others) were picked by
 // timing the 1024x1024x80 step:
 //   trajectory  tiles of 32 i by 4 levels, 7 blocks of 128 threads: 9.54 ms
