@@ -118,15 +118,29 @@ struct WindLayout {
   static constexpr bool soa = PREC == kMixed;
 };
 
-// offsets into the extended, the (ni,nj,nk) and the Adz_wpxyz arrays; the
-// first two volumes are below 2^31 (adzc_setup refuses larger tiles)
+// offsets into the extended, the (ni,nj,nk) and the Adz_wpxyz arrays, in 32
+// bits (the first two volumes are below 2^31: adzc_setup refuses larger tiles)
+// or, I = long long, in 64.  The staged kernels take 32 bits (all in 64 bits:
+// MIXED step 2 % slower at 128 x 128 x 40, 4 % at 512 x 512 x 60).  The direct sets kernels
+// take 64, written out from ni and nj: ptxas then needs 80 registers instead
+// of 96 for FP64 and spills 16 bytes instead of 88 for REF32 (8 clipped
+// fields at 512 x 512 x 60 in REF32 3.27 ms, 3.70 in 32 bits; FP64 2 fields 1.28,
+// 1.37; MIXED 2 fields 0.816, 0.852)
+template <typename I = int>
 __device__ __forceinline__ long long ext_index(const DGrid& g, int i, int j, int k) {
-  return (i - g.lminx) + (j - g.lminy) * g.nit + (k - 1) * (int)g.nij;
+  return (I)(i - g.lminx) + (I)(j - g.lminy) * g.nit + (k - 1) * (I)g.nij;
 }
+template <typename I = int>
 __device__ __forceinline__ long long arr_index(const DGrid& g, int i, int j, int k) {
+  if (sizeof(I) == 8) return (I)(i - 1) + (I)(j - 1) * g.ni + (I)(k - 1) * g.ni * g.nj;
   return (i - 1) + (j - 1) * g.ni + (k - 1) * g.nxy;
 }
+template <typename I = int>
 __device__ __forceinline__ long long wp_index(const DGrid& g, int i, int j, int k, int c) {
+  if (sizeof(I) == 8) {
+    const I nx = g.ni + 4, ny = g.nj + 4;
+    return (I)(i + 1) + (I)(j + 1) * nx + (I)(k - 1) * nx * ny + (I)(c - 1) * nx * ny * g.nk;
+  }
   return ((i + 1) + (j + 1) * g.wnx + (k - 1) * g.wnxy) + (c - 1) * g.wcomp;
 }
 __device__ __forceinline__ double dmin_(double a, double b) { return a < b ? a : b; }
@@ -294,7 +308,7 @@ __device__ __forceinline__ double zindx_t(const DGrid& g, double posz) {
 // stencil of a cell (ix local, x as in the ext array) stays inside the array
 __device__ __forceinline__ bool stencil_ok(const DGrid& g, int off) {
   // off = corner offset relative to cell (1,1,1): recover corner (i,j) in ext coords
-  const long long e = (long long)off + ext_index(g, 1, 1, 1);
+  const long long e = (long long)off + ext_index<long long>(g, 1, 1, 1);
   const long long plane = g.nij;
   long long k = e >= 0 ? e / plane : -1;
   const long long r = e - k * plane;
@@ -667,12 +681,12 @@ __device__ __forceinline__ T ld_traj(const T* p) {
   return *p;
 }
 
-template <int PREC, bool CG = false>
+template <int PREC, bool CG = false, typename I = int>
 __device__ __forceinline__ void set_position(const DGrid& g, const SetArgs& a, int set, int i, int j, int k, double& px,
                                              double& py, double& pz) {
   using F = typename Types<PREC>::F;
   const double aa = -0.0625, bb = 0.5625, half = 0.5;
-  const double* Wx = a.wpxyz + wp_index(g, i, j, k, 1);
+  const double* Wx = a.wpxyz + wp_index<I>(g, i, j, k, 1);
   const double* Wy = Wx + g.wcomp;
   const double* Wz = Wy + g.wcomp;
 #define LX(o) ld_traj<double, CG>(Wx + (o))
@@ -680,7 +694,7 @@ __device__ __forceinline__ void set_position(const DGrid& g, const SetArgs& a, i
 #define LZ(o) ld_traj<double, CG>(Wz + (o))
   if (set == 0) {
     if (PREC == kRef32) {
-      const long long ar = arr_index(g, i, j, k);
+      const long long ar = arr_index<I>(g, i, j, k);
       px = a.pxyzm[3 * ar]; py = a.pxyzm[3 * ar + 1]; pz = a.pxyzm[3 * ar + 2];
     } else {
       px = dmin_(dmax_(LX(0), g.imnx), g.imxx);
@@ -702,9 +716,9 @@ __device__ __forceinline__ void set_position(const DGrid& g, const SetArgs& a, i
     return;
   }
   // set T: Adz_pb
-  const F* wd = (const F*)a.wdep + arr_index(g, i, j, k);
+  const F* wd = (const F*)a.wdep + arr_index<I>(g, i, j, k);
   const int nk = g.nk;
-  const F* zd = (const F*)a.zdt0 + ext_index(g, i, j, k);
+  const F* zd = (const F*)a.zdt0 + ext_index<I>(g, i, j, k);
   const int p = g.wnxy, q = g.nxy;
 #define WD(o) ld_traj<F, CG>(wd + (o))
   double xt, yt, ztv;
@@ -762,15 +776,15 @@ __device__ __forceinline__ double fabs_(double x) { return fabs(x); }
 
 // PERT: the mcrhsint perturbation is set (a.pert); a separate instantiation,
 // so the common path carries none of it
-template <int PREC, bool CG = false, bool PERT = false>
+template <int PREC, bool CG = false, bool PERT = false, typename I = long long>
 __device__ __forceinline__ void set_point(const DGrid& g, int set, const SetArgs& a, const FieldPtrs& fp, int i,
                                           int j, int k) {
   using F = typename Types<PREC>::F;
   const DZtab& lv = (set == 3) ? g.tab_t : g.tab_m;
-  const long long e111 = ext_index(g, 1, 1, 1);
+  const long long e111 = ext_index<I>(g, 1, 1, 1);
   double px, py, pz;
-  set_position<PREC, CG>(g, a, set, i, j, k, px, py, pz);
-  const long long e = ext_index(g, i, j, k);
+  set_position<PREC, CG, I>(g, a, set, i, j, k, px, py, pz);
+  const long long e = ext_index<I>(g, i, j, k);
   if (PREC == kMixed) {
     WF w;
     coef_mixed(w, px, py, pz, lv);
@@ -1568,11 +1582,15 @@ cudaError_t launch_tricub_set(const DGrid& g, int set, int i0, int nx, int j0, i
                               const SetArgs& a, const FieldPtrs& fp, cudaStream_t s) {
   const long long n = (long long)nx * ny * nz;
   if (n <= 0) return cudaSuccess;
-  if constexpr (PREC != kRef32) {
-    if (!a.pert) {
-      SetParts sp{};
-      sp.n = 1;
-      sp.p[0] = SetPart{fp, set, i0, nx, j0, ny, k0, nz, 0};
+  // REF32: the kernel of several parts spills 16 bytes, k_tricub_set 88 (8 clipped
+  // fields at 160 x 150 x 60 308 us, 338), but its parameters of 5 KB lengthen a
+  // launch by 1 to 1.5 us (2 fields at 48 x 40 x 20 take 12)
+  if (PREC == kRef32 ? n * fp.nf >= 400000 : !a.pert) {
+    SetParts sp{};
+    sp.n = 1;
+    sp.p[0] = SetPart{fp, set, i0, nx, j0, ny, k0, nz, 0};
+    if constexpr (PREC == kRef32) return launch_tricub_parts<PREC>(g, a, sp, s);
+    else {
       const SetParts st = st_take_parts<PREC>(sp);
       if (st.n > 0) return st_launch_sets<PREC>(g, a, st, s);
     }

@@ -613,10 +613,10 @@ __global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MI
 
 // ---------------------------------------------------------------------------
 // position sets
-template <int PREC>
+template <int PREC>  // 32-bit offsets: in 64 bits the FP64 kernel spills and is 4 % slower
 __device__ __noinline__ void set_point_direct(const DGrid* g, int set, const SetArgs* a, const FieldPtrs* fp, int i,
                                               int j, int k) {
-  set_point<PREC, false, false>(*g, set, *a, *fp, i, j, k);
+  set_point<PREC, false, false, int>(*g, set, *a, *fp, i, j, k);
 }
 
 // the fields of the position sets' parts on tiles of 32 i x TJ j x TK k
