@@ -24,18 +24,30 @@ namespace adz {
 
 // ---------------------------------------------------------------------------
 // a tile of 32 x TJ x TK points, MINB resident blocks, and room for a box of
-// RP cells in x (RP a multiple of 32 four-byte or 16 eight-byte elements), BY
-// rows and BZ planes
-template <int TJ_, int TK_, int MINB_, int RP_, int BY_, int BZ_>
+// BY rows by BZ planes of RP cells in x (RP a multiple of 32 four-byte or 16
+// eight-byte elements).  DYN: the room is for any ny rows by nz planes with ny
+// * nz <= BY * BZ, the plane pitch (ny rows) being known at run time only.  A
+// sheared flow needs many rows and few planes, a scattered one near the ground
+// many planes; points left out go to the direct code, which is slow here (the
+// boxes leave it little L1).  At 512 x 512 x 60, gyres of 24 cells at Courant
+// number 1.9, two updates: FP64 4.24 ms with the fixed split, 2.96 with any,
+// direct 4.04; REF32 3.07, 2.21, 3.10; in smooth flows the same within 2 %.
+// The pitch costs MIXED's kernels a register that they do not have (2 to 7 %
+// in smooth flows, and two pitches known at compile time 4 to 6 %), so only
+// its tolerance kernel, with 80 registers, takes it
+template <int TJ_, int TK_, int MINB_, int RP_, int BY_, int BZ_, bool DYN_ = false>
 struct StShape {
   static constexpr int TJ = TJ_, TK = TK_, MINB = MINB_, RP = RP_, BY = BY_, BZ = BZ_;
-  static constexpr int NT = 32 * TJ * TK, PP = RP * BY, BOX = PP * BZ;
+  static constexpr int NT = 32 * TJ * TK, ROWS = BY * BZ, BOX = RP * ROWS;
+  static constexpr bool DYN = DYN_;
+  static_assert(ROWS < 256, "StCopy::plan divides by multiplication");
 };
 // trajectory.  MIXED: three component boxes per block; two updates at 1024 x
 // 1024 x 80 6.89 ms, direct 9.57 (4 x 4 points at 2 blocks 2 % slower, 4 x 2
-// points 0.5 %, 3 x 4 points 10 %, 80 registers instead of 64 3 %).  The
-// iteration to a tolerance takes 3 blocks (80 registers): the first step of a
-// run at 768 x 640 x 80 8.77 ms, 9.07 at 4 blocks, 9.65 with the direct kernel.
+// points 0.5 %, 3 x 4 points 10 %, 80 registers instead of 64 3 %).
+// The iteration to a tolerance takes 3 blocks (80 registers): the first step
+// of a run at 768 x 640 x 80 8.77 ms, 9.07 at 4 blocks, 9.65 with the direct kernel
+// (boxes of 96 rows leave less L1: 4 to 13 % slower).
 // FP64: one box of interleaved (u, v, w) cells; 1024 x 512 x 80 6.01 ms,
 // direct 8.43 (2 x 4 points at 2 blocks 6.20); REF32, the same box of FP32
 // cells at 4 blocks (80 registers), 5.81, direct 6.25
@@ -44,9 +56,13 @@ struct TrajBox;
 template <>
 struct TrajBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
 template <>
-struct TrajBox<kFp64> : StShape<3, 2, 3, 48, 8, 8> {};
+struct TrajBox<kFp64> : StShape<3, 2, 3, 48, 8, 8, true> {};
 template <>
-struct TrajBox<kRef32> : StShape<3, 2, 4, 64, 8, 8> {};
+struct TrajBox<kRef32> : StShape<3, 2, 4, 64, 7, 10, true> {};
+struct TolBox : StShape<2, 4, 3, 64, 7, 10, true> {};
+// the shape of a trajectory kernel and of its launch
+template <int PREC, bool TOL>
+using TrajShape = typename std::conditional<TOL, TolBox, TrajBox<PREC>>::type;
 template <int PREC>
 struct SetBox;
 // 8 fields of set t at 1024 x 1024 x 80: 7.93 ms, direct 11.19 (rows that are
@@ -54,9 +70,11 @@ struct SetBox;
 // points 8.59
 template <>
 struct SetBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
-// FP64, 8 fields at 1024 x 512 x 80: 7.38 ms, direct 9.08
+// FP64, 8 fields at 1024 x 512 x 80: 7.38 ms, direct 9.08 (7 rows by 11 planes).
+// 8 clipped fields in the sheared flow above: 5.61 ms with 7 by 11, 4.02 with 8
+// by 10, direct 5.11; in a smooth one 3.25, 3.29, 3.61 (8 by 11 spills: 3.47)
 template <>
-struct SetBox<kFp64> : StShape<2, 4, 2, 48, 7, 11> {};
+struct SetBox<kFp64> : StShape<2, 4, 2, 48, 8, 10> {};
 constexpr int kStRing = 3;  // boxes in flight of the sets kernel
 // fields from which a part of a sets launch is staged: placing and filling
 // the boxes costs about what two fields gain (MIXED at 1024 x 1024 x 80, 2
@@ -68,6 +86,7 @@ constexpr int kStMinFields = 3, kStQvMinFields = 2;
 // a staged box: first cell in the extended array, extents in cells
 struct StBox {
   int ox, oy, oz, nx, ny, nz;
+  int pp;  // plane pitch
 };
 
 // the cell of a position: stencil corner column and row (0-based in the
@@ -126,7 +145,7 @@ __device__ __forceinline__ void st_reduce(int* red, bool use, const Cell& c) {
 // cells; empty when there is no stencil.  MARGIN: with a cell around them
 template <class C, bool MARGIN>
 __device__ __forceinline__ StBox st_box(const DGrid& g, const int* red, int al) {
-  StBox b{0, 0, 0, 0, 0, 0};
+  StBox b{0, 0, 0, 0, 0, 0, 0};
   int x0 = red[0], y0 = red[1], z0 = red[2];
   if (x0 == 0x7fffffff) return b;
   int x1 = 4 - red[3], y1 = 4 - red[4], z1 = 1 - red[5];
@@ -140,18 +159,26 @@ __device__ __forceinline__ StBox st_box(const DGrid& g, const int* red, int al) 
   }
   b.ox = (x1 - (x0 & ~(al - 1)) > C::RP ? imax_(x0, (x0 + x1 - C::RP) / 2) : x0) & ~(al - 1);
   b.nx = imin_(x1 - b.ox, C::RP);
-  b.oy = y1 - y0 > C::BY ? (y0 + y1 - C::BY) / 2 : y0;
-  b.ny = imin_(y1 - b.oy, C::BY);
-  b.oz = z1 - z0 > C::BZ ? (z0 + z1 - C::BZ) / 2 : z0;
-  b.nz = imin_(z1 - b.oz, C::BZ);
+  b.ny = y1 - y0;
+  b.nz = z1 - z0;
+  if (!C::DYN) {
+    b.ny = imin_(b.ny, C::BY);
+    b.nz = imin_(b.nz, C::BZ);
+  } else if (b.ny * b.nz > C::ROWS) {  // BY rows, or those that the planes leave
+    b.ny = imin_(b.ny, imax_(C::BY, C::ROWS / b.nz));
+    b.nz = imin_(b.nz, C::ROWS / b.ny);
+  }
+  b.pp = (C::DYN ? b.ny : C::BY) * C::RP;
+  b.oy = (y0 + y1 - b.ny) / 2;
+  b.oz = (z0 + z1 - b.nz) / 2;
   return b;
 }
 
 // the reduced stencils span more than a box of shape C (uniform over the block)
 template <class C>
 __device__ __forceinline__ bool st_overflow(const int* red, int al) {
-  return red[0] != 0x7fffffff && (4 - red[3] - (red[0] & ~(al - 1)) > C::RP || 4 - red[4] - red[1] > C::BY ||
-                                  1 - red[5] - red[2] > C::BZ);
+  const int nx = 4 - red[3] - (red[0] & ~(al - 1)), ny = 4 - red[4] - red[1], nz = 1 - red[5] - red[2];
+  return red[0] != 0x7fffffff && (nx > C::RP || (C::DYN ? ny * nz > C::ROWS : ny > C::BY || nz > C::BZ));
 }
 
 template <int BYTES>
@@ -178,7 +205,7 @@ struct StCopy {
   static constexpr int CH = 16 / sizeof(T);
   static constexpr int LPR = C::RP / CH <= 16 ? 16 : 32;   // lanes of a row (vec)
   static constexpr int VR = C::NT / LPR, ER = C::NT / 32;  // rows of a pass
-  static constexpr int SLOTS = (C::BY * C::BZ + VR - 1) / VR;
+  static constexpr int SLOTS = (C::ROWS + VR - 1) / VR;
   static_assert(C::RP % CH == 0 && C::RP / CH <= 32, "box shape");
   int off[SLOTS], dst[SLOTS];  // vec: source and shared offsets, dst < 0 for none
   float inv;                   // 1 / rows of a plane
@@ -189,10 +216,10 @@ struct StCopy {
 #pragma unroll
     for (int t = 0; t < SLOTS; t++) {
       const int r = r0 + t * VR;
-      // r < 256 and ny <= 16: the half keeps the product clear of the next integer
+      // r < 256 and ny < 128: the half keeps the product clear of the next integer
       const int z = (int)(((float)r + 0.5f) * inv), y = r - z * b.ny;
       off[t] = z * (int)g.nij + y * g.nit + c;
-      dst[t] = r < rows ? z * C::PP + y * C::RP + c : -1;
+      dst[t] = r < rows ? z * b.pp + y * C::RP + c : -1;
     }
   }
   __device__ __forceinline__ void copy(T* sm, const T* __restrict__ a, const StBox& b, const DGrid& g,
@@ -208,7 +235,7 @@ struct StCopy {
       for (int r = threadIdx.x >> 5; r < rows; r += ER) {
         const int z = (int)(((float)r + 0.5f) * inv), y = r - z * b.ny;
         const T* s = base + (z * (int)g.nij + y * g.nit + lane);
-        T* d = sm + z * C::PP + y * C::RP + lane;
+        T* d = sm + z * b.pp + y * C::RP + lane;
 #pragma unroll
         for (int x = 0; x < C::RP; x += 32)
           if (lane + x < b.nx) cp_async<(int)sizeof(T)>(d + x, s + x);
@@ -228,7 +255,7 @@ __device__ __forceinline__ void st_fill3(T* sm, const T* __restrict__ a, const S
   for (int r = threadIdx.x >> 5; r < rows; r += C::NT / 32) {
     const int z = (int)(((float)r + 0.5f) * inv), y = r - z * b.ny;
     const T* s = base + 3 * (z * g.nij + y * g.nit);
-    T* d = sm + 3 * (z * C::PP + y * C::RP);
+    T* d = sm + 3 * (z * b.pp + y * C::RP);
     if (vec) {
 #pragma unroll
       for (int c = 0; c < 3 * C::RP; c += 32 * CH)
@@ -240,27 +267,28 @@ __device__ __forceinline__ void st_fill3(T* sm, const T* __restrict__ a, const S
 }
 
 // ---------------------------------------------------------------------------
-// sums over a staged box; s: the stencil corner on plane iz0, d0 and d3 the
-// offsets of the lower outer and the upper outer plane from s (those of the
-// inner planes where z is linear)
-template <int RP, int PP>
-__device__ __forceinline__ float st_interp1_mixed(const float* s, int d0, int d3, const float* cx, const float* cy,
-                                                  const float* cz) {
+// sums over a staged box; s: the stencil corner on plane iz0, pp, d0 and d3
+// the offsets of the next plane, the lower outer and the upper outer one from s
+// (those of the inner planes where z is linear)
+template <int RP>
+__device__ __forceinline__ float st_interp1_mixed(const float* s, int pp, int d0, int d3, const float* cx,
+                                                  const float* cy, const float* cz) {
   const float* p0 = s + d0;
   const float* p1 = s;
+  const float* p2 = s + pp;
   const float* p3 = s + d3;
   const float2 cz0 = f2(cz[0], cz[0]), cz1 = f2(cz[1], cz[1]);
   const float2 cz2 = f2(cz[2], cz[2]), cz3 = f2(cz[3], cz[3]);
   float2 ya = f2(0.f, 0.f), yb = f2(0.f, 0.f);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    const int o = r * RP, q = o + PP;
+    const int o = r * RP;
     float2 za = __fmul2_rn(f2(p0[o], p0[o + 1]), cz0);
     float2 zb = __fmul2_rn(f2(p0[o + 2], p0[o + 3]), cz0);
     za = __ffma2_rn(f2(p1[o], p1[o + 1]), cz1, za);
     zb = __ffma2_rn(f2(p1[o + 2], p1[o + 3]), cz1, zb);
-    za = __ffma2_rn(f2(p1[q], p1[q + 1]), cz2, za);
-    zb = __ffma2_rn(f2(p1[q + 2], p1[q + 3]), cz2, zb);
+    za = __ffma2_rn(f2(p2[o], p2[o + 1]), cz2, za);
+    zb = __ffma2_rn(f2(p2[o + 2], p2[o + 3]), cz2, zb);
     za = __ffma2_rn(f2(p3[o], p3[o + 1]), cz3, za);
     zb = __ffma2_rn(f2(p3[o + 2], p3[o + 3]), cz3, zb);
     const float2 cyr = f2(cy[r], cy[r]);
@@ -272,12 +300,13 @@ __device__ __forceinline__ float st_interp1_mixed(const float* s, int d0, int d3
   return x.x + x.y;
 }
 
-template <int RP, int PP>
-__device__ __forceinline__ void st_mono_mixed(const float* s, int d0, int d3, float fx, float fy, float dz,
+template <int RP>
+__device__ __forceinline__ void st_mono_mixed(const float* s, int pp, int d0, int d3, float fx, float fy, float dz,
                                               const float* cx, const float* cy, const float* cz, float& d, float& lin,
                                               float& mn, float& mx) {
   const float* p0 = s + d0;
   const float* p1 = s;
+  const float* p2 = s + pp;
   const float* p3 = s + d3;
   const float2 cz0 = f2(cz[0], cz[0]), cz1 = f2(cz[1], cz[1]);
   const float2 cz2 = f2(cz[2], cz[2]), cz3 = f2(cz[3], cz[3]);
@@ -286,9 +315,9 @@ __device__ __forceinline__ void st_mono_mixed(const float* s, int d0, int d3, fl
   float lo = 3.402823466e38f, hi = -3.402823466e38f;
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    const int o = r * RP, q = o + PP;
+    const int o = r * RP;
     const float2 a1 = f2(p1[o], p1[o + 1]), b1 = f2(p1[o + 2], p1[o + 3]);
-    const float2 a2 = f2(p1[q], p1[q + 1]), b2 = f2(p1[q + 2], p1[q + 3]);
+    const float2 a2 = f2(p2[o], p2[o + 1]), b2 = f2(p2[o + 2], p2[o + 3]);
     float2 za = __fmul2_rn(f2(p0[o], p0[o + 1]), cz0);
     float2 zb = __fmul2_rn(f2(p0[o + 2], p0[o + 3]), cz0);
     za = __ffma2_rn(a1, cz1, za);
@@ -317,10 +346,11 @@ __device__ __forceinline__ void st_mono_mixed(const float* s, int d0, int d3, fl
 }
 
 // interp1_exact
-template <typename T, int RP, int PP>
-__device__ __forceinline__ double st_interp_exact(const T* s, int d0, int d3, const double* c) {
+template <typename T, int RP>
+__device__ __forceinline__ double st_interp_exact(const T* s, int pp, int d0, int d3, const double* c) {
   const T* p0 = s + d0;
   const T* p1 = s;
+  const T* p2 = s + pp;
   const T* p3 = s + d3;
   double ya[4];
 #pragma unroll
@@ -330,7 +360,7 @@ __device__ __forceinline__ double st_interp_exact(const T* s, int d0, int d3, co
       const int o = r * RP + x;
       double za = (double)p0[o] * c[8];
       za = fma((double)p1[o], c[9], za);
-      za = fma((double)p1[o + PP], c[10], za);
+      za = fma((double)p2[o], c[10], za);
       za = fma((double)p3[o], c[11], za);
       ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
     }
@@ -339,10 +369,11 @@ __device__ __forceinline__ double st_interp_exact(const T* s, int d0, int d3, co
 }
 
 // one component of interp3_exact, from cells of three interleaved values
-template <typename T, int RP, int PP>
-__device__ __forceinline__ double st_interp3_exact(const T* s, int d0, int d3, const double* c) {
+template <typename T, int RP>
+__device__ __forceinline__ double st_interp3_exact(const T* s, int pp, int d0, int d3, const double* c) {
   const T* p0 = s + 3 * d0;
   const T* p1 = s;
+  const T* p2 = s + 3 * pp;
   const T* p3 = s + 3 * d3;
   double ya[4];
 #pragma unroll
@@ -352,7 +383,7 @@ __device__ __forceinline__ double st_interp3_exact(const T* s, int d0, int d3, c
       const int o = 3 * (r * RP + x);
       double za = (double)p0[o] * c[8];
       za = fma((double)p1[o], c[9], za);
-      za = fma((double)p1[o + 3 * PP], c[10], za);
+      za = fma((double)p2[o], c[10], za);
       za = fma((double)p3[o], c[11], za);
       ya[x] = (r == 0) ? za * c[4] : fma(za, c[4 + r], ya[x]);
     }
@@ -364,11 +395,12 @@ __device__ __forceinline__ double st_interp3_exact(const T* s, int d0, int d3, c
 }
 
 // interp_mono_exact with the 4-row box
-template <typename T, int RP, int PP>
-__device__ __forceinline__ void st_mono_exact(const T* s, int d0, int d3, const double* c, double& d, double& lin, T& mn,
-                                              T& mx) {
+template <typename T, int RP>
+__device__ __forceinline__ void st_mono_exact(const T* s, int pp, int d0, int d3, const double* c, double& d,
+                                              double& lin, T& mn, T& mx) {
   const T* p0 = s + d0;
   const T* p1 = s;
+  const T* p2 = s + pp;
   const T* p3 = s + d3;
   double ya[4], vyl[4];
   T mi[4], ma[4];  // the bounds of values of type T
@@ -377,7 +409,7 @@ __device__ __forceinline__ void st_mono_exact(const T* s, int d0, int d3, const 
 #pragma unroll
     for (int x = 0; x < 4; x++) {
       const int o = r * RP + x;
-      const T t1 = p1[o], t2 = p1[o + PP];
+      const T t1 = p1[o], t2 = p2[o];
       const double v0 = (double)p0[o], v1 = (double)t1, v2 = (double)t2, v3 = (double)p3[o];
       double za = v0 * c[8];
       if (r == 0) {
@@ -442,24 +474,24 @@ __device__ __noinline__ int traj_update_direct(const DGrid* g, const TrajArgs* a
 }
 
 // departure winds at (px, py, pz) from the staged boxes
-template <int PREC>
+template <int PREC, class C>
 __device__ __forceinline__ void st_winds(const DGrid& g, const typename Types<PREC>::F* sm, const StBox& b,
                                          const StCell& c, double px, double py, double pz, double& ud, double& vd,
                                          double& wd) {
   using F = typename Types<PREC>::F;
-  using C = TrajBox<PREC>;
-  constexpr int RP = C::RP, PP = C::PP;
-  const int d0 = c.zl ? 0 : -PP, d3 = c.zl ? PP : 2 * PP;
-  const int o = (c.iz0 - b.oz) * PP + (c.cj - b.oy) * RP + (c.ci - b.ox);
+  constexpr int RP = C::RP;
+  const int pp = C::DYN ? b.pp : C::BY * RP;
+  const int d0 = c.zl ? 0 : -pp, d3 = c.zl ? pp : 2 * pp;
+  const int o = (c.iz0 - b.oz) * pp + (c.cj - b.oy) * RP + (c.ci - b.ox);
   if constexpr (PREC == kMixed) {
     const int ix = c.ci - g.tab_m.offi + 1 + g.lminx, iy = c.cj - g.tab_m.offj + 1 + g.lminy;
     const float fx = (float)(px - ix), fy = (float)(py - iy), dz = (float)(pz - (c.iz0 + 1));
     float cx[4], cy[4], cz[4];
     st_weights(g.tab_m, c.iz0, c.zl, fx, fy, dz, cx, cy, cz);
     const float* s = sm + o;
-    ud = st_interp1_mixed<RP, PP>(s, d0, d3, cx, cy, cz);
-    vd = st_interp1_mixed<RP, PP>(s + C::BOX, d0, d3, cx, cy, cz);
-    wd = st_interp1_mixed<RP, PP>(s + 2 * C::BOX, d0, d3, cx, cy, cz);
+    ud = st_interp1_mixed<RP>(s, pp, d0, d3, cx, cy, cz);
+    vd = st_interp1_mixed<RP>(s + C::BOX, pp, d0, d3, cx, cy, cz);
+    wd = st_interp1_mixed<RP>(s + 2 * C::BOX, pp, d0, d3, cx, cy, cz);
   } else {
     double cf[20];
     int off;
@@ -467,9 +499,9 @@ __device__ __forceinline__ void st_winds(const DGrid& g, const typename Types<PR
     else coef_f64pos(cf, off, px, py, pz, g.tab_m);
     const F* s = sm + 3 * o;
     // Tricublin_zyx3_n returns ``real`` (F)
-    ud = (double)(F)st_interp3_exact<F, RP, PP>(s, d0, d3, cf);
-    vd = (double)(F)st_interp3_exact<F, RP, PP>(s + 1, d0, d3, cf);
-    wd = (double)(F)st_interp3_exact<F, RP, PP>(s + 2, d0, d3, cf);
+    ud = (double)(F)st_interp3_exact<F, RP>(s, pp, d0, d3, cf);
+    vd = (double)(F)st_interp3_exact<F, RP>(s + 1, pp, d0, d3, cf);
+    wd = (double)(F)st_interp3_exact<F, RP>(s + 2, pp, d0, d3, cf);
   }
 }
 
@@ -483,16 +515,22 @@ __device__ __forceinline__ void st_winds(const DGrid& g, const typename Types<PR
 // (a margin of levels only: 8.98 against 8.76 ms).
 // Else a.niter updates.
 template <int PREC, bool TOL>
-__global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MINB)
+__global__ void __launch_bounds__(TrajShape<PREC, TOL>::NT, TrajShape<PREC, TOL>::MINB)
     k_traject_st(const __grid_constant__ DGrid g, const __grid_constant__ TrajArgs a, int i0, int nx, int j0, int ny,
                  double tol, int maxit, unsigned char* iters, unsigned long long* stats,
                  const __grid_constant__ GuessStart gs) {
   using F = typename Types<PREC>::F;
-  using C = TrajBox<PREC>;
+  using C = TrajShape<PREC, TOL>;
   constexpr int TK = C::TK, TJ = C::TJ, AL = 16 / sizeof(F);
   extern __shared__ uint4 st_dyn[];
   F* sm = reinterpret_cast<F*>(st_dyn);
   __shared__ int red[6];
+  // the box in shared memory leaves more registers to the sums (FP64: nothing
+  // spills, else 16 bytes); MIXED keeps it in registers (96 bytes instead of 32)
+  constexpr bool RB = PREC == kMixed;
+  __shared__ StBox sbox;
+  StBox rbox;
+  StBox& box = RB ? rbox : sbox;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = i0 + (int)blockIdx.x * 32 + lane;
   const int k = a.k00 + (int)blockIdx.y * TK + w % TK;
@@ -514,28 +552,29 @@ __global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MI
       warm_start<PREC>(g, a, i, j, k, s.px, s.py, s.pz);
     }
   }
-  StBox box;
   auto place = [&](bool use, const StCell& c) {  // place the box and start its copies
     st_reduce(red, use, c);
     __syncthreads();
-    box = st_box<C, TOL>(g, red, vec ? AL : 1);
+    StBox b = st_box<C, TOL>(g, red, vec ? AL : 1);
     // FP64, REF32: where more than a quarter of the points would be left out
     // (strong shear inside the tile), the direct code takes them all (83 x 192 x
     // 59 at Courant numbers up to 2: 0.217 against 0.25 ms).  In the MIXED
     // kernel the test costs more in spills (7.8 against 6.9 ms) than it saves
     if constexpr (PREC != kMixed)
-      if (st_overflow<C>(red, vec ? AL : 1) && __syncthreads_count(use && !st_in_box(box, c)) > C::NT / 4) {
-        box.nx = 0;
+      if (st_overflow<C>(red, vec ? AL : 1) && __syncthreads_count(use && !st_in_box(b, c)) > C::NT / 4) {
+        b.nx = 0;
+        if (RB || threadIdx.x == 0) box = b;
         return;
       }
+    if (RB || threadIdx.x == 0) box = b;  // seen after the barrier that ends the copies
     const F* uvw = (const F*)a.uvw_d;
     if constexpr (PREC == kMixed) {
       StCopy<F, C> cp;
-      cp.plan(box, g, vec);
+      cp.plan(b, g, vec);
 #pragma unroll
-      for (int q = 0; q < 3; q++) cp.copy(sm + q * C::BOX, uvw + q * g.nij * g.nk, box, g, vec);
+      for (int q = 0; q < 3; q++) cp.copy(sm + q * C::BOX, uvw + q * g.nij * g.nk, b, g, vec);
     } else {
-      st_fill3<F, C>(sm, uvw, box, g, vec);
+      st_fill3<F, C>(sm, uvw, b, g, vec);
     }
     cp_async_commit();
   };
@@ -555,7 +594,7 @@ __global__ void __launch_bounds__(TrajBox<PREC>::NT, TOL ? 3 : TrajBox<PREC>::MI
       const double qx = s.px, qy = s.py, qz = s.pz;
       if (ok && st_in_box(box, c)) {
         double ud, vd;
-        st_winds<PREC>(g, sm, box, c, s.px, s.py, s.pz, ud, vd, s.wd);
+        st_winds<PREC, C>(g, sm, box, c, s.px, s.py, s.pz, ud, vd, s.wd);
         st = traj_advance<PREC>(g, a, i, j, k, s.ua, s.va, s.wa, ud, vd, s.wd, s.px, s.py, s.pz, s.xm, s.ym, s.w3);
       } else {
         TrajState t = s;
@@ -628,7 +667,7 @@ __global__ void __launch_bounds__(SetBox<PREC>::NT, SetBox<PREC>::MINB)
     k_sets_st(const __grid_constant__ DGrid g, const __grid_constant__ SetArgs a, const __grid_constant__ SetParts sp) {
   using F = typename Types<PREC>::F;
   using C = SetBox<PREC>;
-  constexpr int TK = C::TK, TJ = C::TJ, RP = C::RP, PP = C::PP, BOX = C::BOX;
+  constexpr int TK = C::TK, TJ = C::TJ, RP = C::RP, BOX = C::BOX;
   extern __shared__ uint4 st_dyn[];
   F* ring = reinterpret_cast<F*>(st_dyn);
   __shared__ int red[6];
@@ -667,8 +706,9 @@ __global__ void __launch_bounds__(SetBox<PREC>::NT, SetBox<PREC>::MINB)
 #pragma unroll
   for (int q = 0; q < kStRing - 1; q++) copy(q, q);
   in = in && st_in_box(box, c);
-  const int o = (c.iz0 - box.oz) * PP + (c.cj - box.oy) * RP + (c.ci - box.ox);
-  const int d0 = c.zl ? 0 : -PP, d3 = c.zl ? PP : 2 * PP;
+  const int pp = C::DYN ? box.pp : C::BY * RP;
+  const int o = (c.iz0 - box.oz) * pp + (c.cj - box.oy) * RP + (c.ci - box.ox);
+  const int d0 = c.zl ? 0 : -pp, d3 = c.zl ? pp : 2 * pp;
   typename std::conditional<PREC == kMixed, float, double>::type cf[20];
   float fx = 0.f, fy = 0.f, dz = 0.f;
   if (in) {
@@ -696,20 +736,20 @@ __global__ void __launch_bounds__(SetBox<PREC>::NT, SetBox<PREC>::MINB)
     if constexpr (PREC == kMixed) {
       if ((fp.mono_mask >> q) & 1u) {
         float d, lin, mn, mx;
-        st_mono_mixed<RP, PP>(s, d0, d3, fx, fy, dz, cf, cf + 4, cf + 8, d, lin, mn, mx);
+        st_mono_mixed<RP>(s, pp, d0, d3, fx, fy, dz, cf, cf + 4, cf + 8, d, lin, mn, mx);
         if ((fp.clip_mask >> q) & 1u) d = fmaxf(mn, fminf(mx, d));
         if (fp.lin[q]) ((float*)fp.lin[q])[e] = fmaxf(mn, fminf(mx, lin));
         if (fp.mn[q]) ((float*)fp.mn[q])[e] = mn;
         if (fp.mx[q]) ((float*)fp.mx[q])[e] = mx;
         ((float*)fp.dst[q])[e] = d;
       } else {
-        ((float*)fp.dst[q])[e] = st_interp1_mixed<RP, PP>(s, d0, d3, cf, cf + 4, cf + 8);
+        ((float*)fp.dst[q])[e] = st_interp1_mixed<RP>(s, pp, d0, d3, cf, cf + 4, cf + 8);
       }
     } else {
       if ((fp.mono_mask >> q) & 1u) {
         double d, lin;
         F mnf, mxf;
-        st_mono_exact<F, RP, PP>(s, d0, d3, cf, d, lin, mnf, mxf);
+        st_mono_exact<F, RP>(s, pp, d0, d3, cf, d, lin, mnf, mxf);
         F df = (F)d, lf = (F)lin;
         if ((fp.clip_mask >> q) & 1u) df = (mnf > ((mxf < df) ? mxf : df)) ? mnf : ((mxf < df) ? mxf : df);
         if (fp.lin[q]) ((F*)fp.lin[q])[e] = (mnf > ((mxf < lf) ? mxf : lf)) ? mnf : ((mxf < lf) ? mxf : lf);
@@ -717,7 +757,7 @@ __global__ void __launch_bounds__(SetBox<PREC>::NT, SetBox<PREC>::MINB)
         if (fp.mx[q]) ((F*)fp.mx[q])[e] = mxf;
         ((F*)fp.dst[q])[e] = df;
       } else {
-        ((F*)fp.dst[q])[e] = (F)st_interp_exact<F, RP, PP>(s, d0, d3, cf);
+        ((F*)fp.dst[q])[e] = (F)st_interp_exact<F, RP>(s, pp, d0, d3, cf);
       }
     }
   }
@@ -791,7 +831,7 @@ __global__ void __launch_bounds__(QvBox::NT, QvBox::MINB)
             int i0, int nx, int j0, int ny, int k0, int nz, int vec) {
   static_assert(PREC == kMixed, "FP32 sums");
   using C = QvBox;
-  constexpr int TK = C::TK, TJ = C::TJ, RP = C::RP, PP = C::PP, BOX = C::BOX;
+  constexpr int TK = C::TK, TJ = C::TJ, RP = C::RP, BOX = C::BOX;
   extern __shared__ uint4 st_dyn[];
   float* ring = reinterpret_cast<float*>(st_dyn);
   __shared__ int red[6];
@@ -836,8 +876,9 @@ __global__ void __launch_bounds__(QvBox::NT, QvBox::MINB)
 #pragma unroll
   for (int q = 0; q < kStRing - 1; q++) copy(q, q);
   in = in && st_in_box(box, cell);
-  const int o = (cell.k0 - box.oz) * PP + (cell.cj - box.oy) * RP + (cell.ci - box.ox);
-  const int p1 = nc * PP, p2 = p1 + nl * PP, p3 = p2 + PP, p4 = p3 + nl * PP, p5 = p4 + nc * PP;
+  const int pp = C::DYN ? box.pp : C::BY * RP;
+  const int o = (cell.k0 - box.oz) * pp + (cell.cj - box.oy) * RP + (cell.ci - box.ox);
+  const int p1 = nc * pp, p2 = p1 + nl * pp, p3 = p2 + pp, p4 = p3 + nl * pp, p5 = p4 + nc * pp;
   const int e = (int)ext_index(g, i, j, k);
   int use = 0, next = kStRing - 1;
 #pragma unroll 1
@@ -895,7 +936,7 @@ SetParts st_take_parts(SetParts& sp) {
 template <int PREC, bool TOL>
 cudaError_t st_launch_traject(const DGrid& g, const TrajArgs& a, int i0, int nx, int j0, int ny, double tol, int maxit,
                               unsigned char* iters, unsigned long long* stats, const GuessStart& gs, cudaStream_t s) {
-  using C = TrajBox<PREC>;
+  using C = TrajShape<PREC, TOL>;
   const int nkp = g.nk - a.k00 + 1;
   if (nx <= 0 || ny <= 0 || nkp <= 0) return cudaSuccess;
   constexpr int smem = 3 * C::BOX * (int)sizeof(typename Types<PREC>::F);
