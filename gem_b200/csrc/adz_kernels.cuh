@@ -1516,7 +1516,7 @@ cudaError_t launch_inittraj(const DGrid& g, float* pxyzm, double* wpxyz, cudaStr
 
 template <int PREC>
 cudaError_t launch_traject(const DGrid& g, const TrajArgs& a, cudaStream_t s) {
-  if (st_grid_ok<PREC>(g, a.k00, g.nj))
+  if (st_traject_ok<PREC, false>(g, a, g.ni, g.nj))
     return st_launch_traject<PREC, false>(g, a, 1, g.ni, 1, g.nj, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
 #if ADZ_TRAJ_TILE_K > 1
   constexpr int TK = ADZ_TRAJ_TILE_K, TI = ADZ_TRAJ_TILE_I;
@@ -1535,7 +1535,7 @@ cudaError_t launch_traject_box(const DGrid& g, const TrajArgs& a, int i0, int nx
   const long long nkp = g.nk - a.k00 + 1, n = (long long)nx * ny * nkp;
   if (n <= 0) return cudaSuccess;
   if (batch_use_tiles(nx, nkp)) {
-    if (st_grid_ok<PREC>(g, a.k00, ny))
+    if (st_traject_ok<PREC, false>(g, a, nx, ny))
       return st_launch_traject<PREC, false>(g, a, i0, nx, j0, ny, 0.0, 0, nullptr, nullptr, GuessStart{}, s);
     const long long nb = (long long)((nx + 31) / 32) * ((nkp + 3) / 4) * ny;
     if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -1564,7 +1564,7 @@ cudaError_t launch_traject_tol(const DGrid& g, const TrajArgs& a, double tol, in
   // bytes gain less (first step of a run at 765 x 640 x 80: 10.33 ms staged, 10.62
   // direct; 768: 8.76 and 9.65)
   if constexpr (PREC == kMixed)
-    if (st_grid_ok<PREC>(g, a.k00, g.nj))
+    if (st_traject_ok<PREC, true>(g, a, g.ni, g.nj))
       return st_launch_traject<PREC, true>(g, a, 1, g.ni, 1, g.nj, tol, maxit, iters, stats, gs, s);
 #if ADZ_TOL_TILES
   const long long nb = (long long)((g.ni + 31) / 32) * ((g.nk - a.k00 + 1 + 3) / 4) * g.nj;
@@ -1582,18 +1582,15 @@ cudaError_t launch_tricub_set(const DGrid& g, int set, int i0, int nx, int j0, i
                               const SetArgs& a, const FieldPtrs& fp, cudaStream_t s) {
   const long long n = (long long)nx * ny * nz;
   if (n <= 0) return cudaSuccess;
+  const SetPart P{fp, set, i0, nx, j0, ny, k0, nz, 0};
   // REF32: the kernel of several parts spills 16 bytes, k_tricub_set 88 (8 clipped
   // fields at 160 x 150 x 60 308 us, 338), but its parameters of 5 KB lengthen a
   // launch by 1 to 1.5 us (2 fields at 48 x 40 x 20 take 12)
-  if (PREC == kRef32 ? n * fp.nf >= 400000 : !a.pert) {
+  if (PREC == kRef32 ? n * fp.nf >= 400000 : !a.pert && st_part_ok<PREC>(g, P, P.nx, P.ny, P.nz)) {
     SetParts sp{};
     sp.n = 1;
-    sp.p[0] = SetPart{fp, set, i0, nx, j0, ny, k0, nz, 0};
-    if constexpr (PREC == kRef32) return launch_tricub_parts<PREC>(g, a, sp, s);
-    else {
-      const SetParts st = st_take_parts<PREC>(sp);
-      if (st.n > 0) return st_launch_sets<PREC>(g, a, st, s);
-    }
+    sp.p[0] = P;
+    return launch_tricub_parts<PREC>(g, a, sp, s);
   }
 #if ADZ_SET_TILE_K > 1
   constexpr int TK = ADZ_SET_TILE_K, TI = 128 / TK;
@@ -1620,16 +1617,16 @@ cudaError_t launch_positions(const DGrid& g, int set, int i0, int nx, int j0, in
 template <int PREC>
 cudaError_t launch_tricub_parts(const DGrid& g, const SetArgs& a, const SetParts& parts, cudaStream_t s) {
   if (parts.n < 1 || parts.n > kMaxParts) return cudaErrorInvalidValue;
-  SetParts sp = parts;
-  if constexpr (PREC != kRef32) {
-    if (!a.pert) {
-      const SetParts st = st_take_parts<PREC>(sp);
-      if (st.n > 0) {
-        const cudaError_t e = st_launch_sets<PREC>(g, a, st, s);
-        if (e != cudaSuccess || sp.n == 0) return e;
-      }
+  SetParts rest;  // the parts of the direct kernel where the staged one takes some
+  const bool some = PREC != kRef32 && !a.pert && st_takes_some<PREC>(g, parts);
+  if constexpr (PREC != kRef32)
+    if (some) {
+      rest = parts;
+      const SetParts st = st_take_parts<PREC>(g, rest);
+      const cudaError_t e = st_launch_sets<PREC>(g, a, st, s);
+      if (e != cudaSuccess || rest.n == 0) return e;
     }
-  }
+  const SetParts& sp = some ? rest : parts;
   long long most = 0;  // blocks of the largest part
   for (int q = 0; q < sp.n; q++) {
 #if ADZ_SET_TILE_K > 1
@@ -1660,7 +1657,7 @@ cudaError_t launch_qv_set(const DGrid& g, int i0, int nx, int j0, int ny, int k0
   const long long n = (long long)nx * ny * nz;
   if (n <= 0) return cudaSuccess;
   if constexpr (PREC == kMixed)
-    if (!a.pert && fp.nf >= kStQvMinFields && (nz + 3) / 4 <= 65535 && (ny + 1) / 2 <= 65535)
+    if (!a.pert && st_qv_ok(fp.nf, nx, ny, nz))
       return st_launch_qv<PREC>(g, i0, nx, j0, ny, k0, nz, a, fp, s);
 #if ADZ_QV_TILES
   const long long nb = (long long)((nx + 31) / 32) * ((nz + 3) / 4) * ny;

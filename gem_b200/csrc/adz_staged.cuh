@@ -40,6 +40,7 @@ struct StShape {
   static constexpr int TJ = TJ_, TK = TK_, MINB = MINB_, RP = RP_, BY = BY_, BZ = BZ_;
   static constexpr int NT = 32 * TJ * TK, ROWS = BY * BZ, BOX = RP * ROWS;
   static constexpr bool DYN = DYN_;
+  static constexpr long long WAVE = 148LL * MINB * NT;  // points of the blocks that run at once
   static_assert(ROWS < 256, "StCopy::plan divides by multiplication");
 };
 // trajectory.  MIXED: three component boxes per block; two updates at 1024 x
@@ -76,12 +77,38 @@ struct SetBox<kMixed> : StShape<2, 4, 4, 64, 7, 10> {};
 template <>
 struct SetBox<kFp64> : StShape<2, 4, 2, 48, 8, 10> {};
 constexpr int kStRing = 3;  // boxes in flight of the sets kernel
+// A launch whose blocks all run at once takes as long as one block, and the
+// staged block's chain is longer, so small launches stay direct (C::WAVE points
+// are one wave).  Staged against direct speed, smooth flow / gyres at Courant
+// number 1.9, at 48 x 40 x 20, 64 x 64 x 24 (98 K points), 30 x 200 x 24 (144 K), 96 x 90 x
+// 40 (346 K):
+//   two updates, MIXED  1.09 / 0.68, 1.15 / 0.83, 1.08 / 0.92, 1.34 / 1.08: one wave
+//                       (152 K)
+//   FP64, DYN           1.11 / 1.19, 1.11 / 1.08, 1.24 / 1.23, 1.30 / 1.33; REF32 1.00 /
+//                       1.11, 1.14 / 1.23, 0.96 / 1.11, 1.10 / 1.17: half a wave (43 K, 57 K)
+//   six from the arrival points, which place their box twice, MIXED 0.57, 1.10,
+//                       0.68, 1.15 (smooth), FP64 0.76, 0.91, 1.07, 1.18: 1.5 waves (227 K,
+//                       128 K).  REF32 0.65, 0.79, 0.72, 0.93, at 512 x 512 x 60 0.95: direct
+//   sets, MIXED         3 fields 0.90 / 0.73, 1.06 / 0.85, 0.98 / 0.91, 1.24 / 1.06; 8 fields
+//                       1.01 / 0.79, 1.29 / 0.94, 1.00 / 0.95, 1.44 / 1.22: one wave, half
+//                       a wave where the rows are copied in 16-byte pieces (all but 30 x
+//                       200), and four waves of points times fields
+//   BICUBH_QV           3 fields 0.95 / 0.85, 1.27 / 0.94, 1.03 / 0.94, 1.34 / 1.16: half a
+//                       wave (57 K)
+// The iteration to a tolerance is staged at every size: from the arrival points
+// 0.97 to 1.20 at those sizes, from a converged start 1.35 to 1.57
+
 // fields from which a part of a sets launch is staged: placing and filling
 // the boxes costs about what two fields gain (MIXED at 1024 x 1024 x 80, 2
-// fields: 3.44 ms staged, 3.36 direct; 5 fields 5.64 and 7.19; FP64 at 1024 x
-// 512 x 80, 2 fields: 3.14 and 2.85, 5 fields 5.07 and 5.95).  The sets of
-// REF32 stay direct (8 fields: 6.88 staged, 6.37 direct)
-constexpr int kStMinFields = 3, kStQvMinFields = 2;
+// fields: 3.44 ms staged, 3.36 direct; 5 fields 5.64 and 7.19), in FP64 with bounds
+// three (1024 x 512 x 80, 3 fields 4.13 and 3.89 ms, 4 4.79 and 4.91; 3 fields
+// without bounds 3.77 and 3.69, at 250 x 60 x 70 110 and 138 us).  The sets of REF32
+// stay direct (8 fields: 6.88 staged, 6.37 direct)
+constexpr int kStQvMinFields = 2;
+template <int PREC>
+bool st_fields_ok(const FieldPtrs& fp) {
+  return fp.nf >= (PREC == kFp64 && fp.mono_mask ? 4 : 3);
+}
 
 // a staged box: first cell in the extended array, extents in cells
 struct StBox {
@@ -902,32 +929,56 @@ __global__ void __launch_bounds__(QvBox::NT, QvBox::MINB)
 }
 
 // ---------------------------------------------------------------------------
-// whether the grid of a launch fits (its y and z extents are below 65536);
-// larger tiles take the direct kernels
-template <int PREC>
-bool st_grid_ok(const DGrid& g, int k00, int ny) {
-  using C = TrajBox<PREC>;
-  return (g.nk - k00 + C::TK) / C::TK <= 65535 && (ny + C::TJ - 1) / C::TJ <= 65535;
+// whether the staged kernel runs the trajectory of nx columns by ny rows: from
+// the sizes above on, and its grid's y and z extents have to be below 65536
+template <int PREC, bool TOL>
+bool st_traject_ok(const DGrid& g, const TrajArgs& a, int nx, int ny) {
+  using C = TrajShape<PREC, TOL>;
+  const long long nk = g.nk - a.k00 + 1, n = (long long)nx * ny * nk;
+  if ((nk + C::TK - 1) / C::TK > 65535 || (ny + C::TJ - 1) / C::TJ > 65535) return false;
+  if (TOL) return true;
+  if (a.cold) return PREC != kRef32 && 2 * n >= 3 * C::WAVE;
+  return n >= (C::DYN ? C::WAVE / 2 : C::WAVE);
 }
-// takes the parts of a sets launch that the staged kernel runs out of sp:
-// those of kStMinFields fields or more whose boxes are alike (each fills at
-// least half of the region that spans the largest; not so the boxes of a
-// band) and whose grid fits
+// whether the staged kernel runs a part of a sets launch: one of enough points
+// and fields whose box is like the launch's largest extents nx, ny, nz (it fills
+// at least half of them; not so the boxes of a band) and whose grid fits
 template <int PREC>
-SetParts st_take_parts(SetParts& sp) {
-  using C = SetBox<PREC>;
-  SetParts st{}, rest{};
-  long long nx = 0, ny = 0, nz = 0;
+bool st_part_ok(const DGrid& g, const SetPart& P, long long nx, long long ny, long long nz) {
+  if constexpr (PREC == kRef32) return false;
+  else {
+    using C = SetBox<PREC>;
+    const long long n = (long long)P.nx * P.ny * P.nz;
+    const bool rows16 = g.nit % (16 / (int)sizeof(typename Types<PREC>::F)) == 0;
+    return st_fields_ok<PREC>(P.fp) && (rows16 ? 2 * n : n) >= C::WAVE && n * P.fp.nf >= 4 * C::WAVE && 2 * n >= nx * ny * nz &&
+           (nz + C::TK - 1) / C::TK <= 65535 && (ny + C::TJ - 1) / C::TJ <= 65535;
+  }
+}
+inline void st_extents(const SetParts& sp, long long& nx, long long& ny, long long& nz) {
+  nx = ny = nz = 0;
   for (int q = 0; q < sp.n; q++) {
     nx = sp.p[q].nx > nx ? sp.p[q].nx : nx;
     ny = sp.p[q].ny > ny ? sp.p[q].ny : ny;
     nz = sp.p[q].nz > nz ? sp.p[q].nz : nz;
   }
-  const bool fits = (nz + C::TK - 1) / C::TK <= 65535 && (ny + C::TJ - 1) / C::TJ <= 65535;
+}
+template <int PREC>
+bool st_takes_some(const DGrid& g, const SetParts& sp) {
+  long long nx, ny, nz;
+  st_extents(sp, nx, ny, nz);
+  for (int q = 0; q < sp.n; q++)
+    if (st_part_ok<PREC>(g, sp.p[q], nx, ny, nz)) return true;
+  return false;
+}
+// takes the parts of a sets launch that the staged kernel runs out of sp
+template <int PREC>
+SetParts st_take_parts(const DGrid& g, SetParts& sp) {
+  SetParts st{}, rest{};
+  long long nx, ny, nz;
+  st_extents(sp, nx, ny, nz);
   for (int q = 0; q < sp.n; q++) {
-    const SetPart& P = sp.p[q];
-    if (fits && P.fp.nf >= kStMinFields && 2LL * P.nx * P.ny * P.nz >= nx * ny * nz) st.p[st.n++] = P;
-    else rest.p[rest.n++] = P;
+    if (st_part_ok<PREC>(g, sp.p[q], nx, ny, nz)) st.p[st.n++] = sp.p[q];
+    else rest.p[rest.n++] = sp.p[q];
   }
   sp = rest;
   return st;
@@ -970,6 +1021,13 @@ cudaError_t st_launch_sets(const DGrid& g, const SetArgs& a, const SetParts& par
   const dim3 grid((nx + 31) / 32 * sp.n, (nz + C::TK - 1) / C::TK, (ny + C::TJ - 1) / C::TJ);
   k_sets_st<PREC><<<grid, C::NT, smem, s>>>(g, a, sp);
   return cudaGetLastError();
+}
+
+// whether the staged kernel runs nf BICUBH_QV fields of nx x ny x nz points
+inline bool st_qv_ok(int nf, int nx, int ny, int nz) {
+  using C = QvBox;
+  return nf >= kStQvMinFields && 2LL * nx * ny * nz >= C::WAVE && (nz + C::TK - 1) / C::TK <= 65535 &&
+         (ny + C::TJ - 1) / C::TJ <= 65535;
 }
 
 template <int PREC>

@@ -12,6 +12,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 SIZES = [(33, 9, 5), (64, 40, 24), (97, 51, 13), (40, 41, 4), (31, 2, 8)]
+# from two waves of blocks on (303104 points in MIXED) every launch is staged
+SIZES += [(97, 51, 62), (33, 400, 24), (2100, 9, 17), (40, 41, 190), (64, 1250, 4)]
 
 
 def _case(prec_name, size, wild, ntr, seed=3):
