@@ -189,3 +189,63 @@ def test_bc_lam_flux_vs_oracle(prec_name, gbpil, psadj):
         assert np.array_equal(_bits(g[w]), _bits(o[w]))
     # the fluxes are not trivially zero: both carry tracer outside the zeroed parts
     assert all(np.nanmax(np.abs(o)) > 0 for o in o_fo + o_fi)
+
+
+# tiles that touch some LAM edges or none, sizes that are no multiples of the
+# kernel's tiles of 32 columns by 4 levels, and a top pilot zone
+@pytest.mark.parametrize("edges,gbpil", [((1, 1, 1, 1), 0), ((1, 1, 1, 1), 4), ((1, 0, 0, 0), 0), ((0, 1, 1, 0), 3),
+                                         ((0, 0, 0, 0), 0)])
+@pytest.mark.parametrize("size", [(48, 40, 20), (67, 45, 13)])
+@pytest.mark.parametrize("prec_name", ["ref32", "fp64", "mixed"])
+def test_bc_lam_flux_edges(prec_name, size, edges, gbpil):
+    """REF32 and FP64 against the restatement; MIXED against the masked tracers
+    interpolated at Adz_pb by adzc_tricub and zeroed, by value."""
+    from gem_b200 import adz as A, synth
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    prec = A.PREC_NAMES[prec_name]
+    dt = A._field_dtype(prec)
+    cfg = synth.config_small(*size)
+    cfg.ntracers, cfg.tracer_kind = 3, "lognormal"
+    inp = synth.make_inputs(cfg, device="cuda", dtype=dt)
+    ad = A.Adz.from_config(cfg, edges=edges, lam_gbpil_t=gbpil)
+    px, wp = ad.new_state(prec)
+    ad.adz_inittraj(prec, px, wp)
+    ad.adz_traject(prec, cfg.dt, inp, px, wp)
+    trs = inp["tracers"]
+    nan = lambda: torch.full(ad.ext_shape, float("nan"), dtype=dt, device="cuda")  # noqa: E731
+    fo, fi = [nan() for _ in trs], [nan() for _ in trs]
+    ad.bc_lam_flux(prec, trs, fo, fi)
+    torch.cuda.synchronize()
+    assert ad.status() == 0
+    if prec != A.MIXED:
+        st = O.Step(cfg, kind="oracle", prec="f32" if prec == A.REF32 else "f64", lam_gbpil_t=gbpil, edges=edges)
+        st.inittraj()
+        st.traject({k: inp[k].cpu().numpy() for k in ("uu_ext", "vv_ext", "ww_ext", "ut0", "vt0", "zdt0")})
+        r_fo, r_fi = st.bc_lam_flux([t.cpu().numpy() for t in trs])
+    else:
+        I, H, p = ad.info, cfg.halo, cfg.pil
+        w, e, s, n = edges
+        i = torch.arange(1 - H, cfg.ni + H + 1, device="cuda").view(1, 1, -1)
+        j = torch.arange(1 - H, cfg.nj + H + 1, device="cuda").view(1, -1, 1)
+        k = torch.arange(1, cfg.nk + 1, device="cuda").view(-1, 1, 1)
+        dom = (i >= (1 if w else -99)) & (i <= (cfg.ni if e else 999)) & (j >= (1 if s else -99)) & (
+            j <= (cfg.nj if n else 999)) & (k > 0)
+        core = dom & (i >= (1 + p if w else -99)) & (i <= (cfg.ni - p if e else 999)) & (
+            j >= (1 + p if s else -99)) & (j <= (cfg.nj - p if n else 999)) & (k >= I.k0t)
+        zero = torch.zeros((), dtype=dt, device="cuda")
+        r_fo, r_fi = [nan() for _ in trs], [nan() for _ in trs]
+        for q, t in enumerate(trs):  # one field at a time: the direct kernel at every size
+            ad.adz_tricub_hlt(prec, A.SET_B, [torch.where(core, t, zero)], [r_fo[q]])
+            ad.adz_tricub_hlt(prec, A.SET_B, [torch.where(dom & ~core, t, zero)], [r_fi[q]])
+        own = (i >= 1) & (i <= cfg.ni) & (j >= 1) & (j <= cfg.nj)
+        low, b = own & (k >= I.k0t), ad.range_mask(A.SET_B, device="cuda")
+        pil = (i <= p * w) | (i >= cfg.ni - p * e + 1) | (j <= p * s) | (j >= cfg.nj - p * n + 1)
+        for q in range(len(trs)):
+            r_fo[q][low & ~pil] = 0.0
+            r_fi[q][(low & pil) | (own & b & (k < I.k0t))] = 0.0
+        r_fo, r_fi = ([t.cpu().numpy() for t in r] for r in (r_fo, r_fi))
+    for got, ref in zip(fo + fi, r_fo + r_fi):
+        assert np.array_equal(got.cpu().numpy(), ref, equal_nan=True)
+    if any(edges):
+        assert all(np.nanmax(np.abs(r)) > 0 for r in r_fo)

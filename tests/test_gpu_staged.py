@@ -1,9 +1,11 @@
 """The step's gather kernels on shared-memory boxes against the direct ones,
 bit for bit (they form the same sums in the same order): trajectories against
-the phased batch plan, the position sets and BICUBH_QV against the same call
-with a zero perturbation pattern, which the direct kernels run.  Sizes at the
-edges of tiles and boxes, rows that are not 16-byte multiples, sources off a
-16-byte boundary, few levels, and flows so scattered that stencils leave their
+the phased batch plan (REF32 against the oracle), the iteration to a tolerance
+against fixed updates, the position sets and BICUBH_QV against the same call
+with a zero perturbation pattern, which the direct kernels run.  Small tiles,
+which the direct kernels take, and sizes at the edges of tiles and boxes, rows
+that are not 16-byte multiples, sources off a 16-byte boundary, few levels,
+flows sheared within a tile, and flows so scattered that stencils leave their
 box or the boxes are placed more than once."""
 import numpy as np
 import pytest
@@ -25,10 +27,17 @@ def _case(prec_name, size, wild, ntr, seed=3):
     cfg = synth.config_small(*size)
     cfg.ntracers, cfg.tracer_kind = ntr, "lognormal"
     inp = synth.make_inputs(cfg, device="cuda", dtype=ft)
-    if wild:  # departure points anywhere within the halo, levels away
+    if wild == "shear":  # gyres of 24 cells, about two cells per step: many rows per tile
+        k, j, i = (torch.arange(n, device="cuda", dtype=torch.float64) for n in inp["uu_ext"].shape)
+        i, j, c = 0.262 * i + 0.1 * k.view(-1, 1, 1), 0.262 * j.view(1, -1, 1), 1.9 * cfg.dx / cfg.dt
+        for key, f in (("uu_ext", torch.sin(j) * torch.cos(i)), ("vv_ext", -torch.cos(j) * torch.sin(i))):
+            inp[key] = (c * f).to(ft).contiguous()
+            inp[key.replace("u_ext", "t0").replace("v_ext", "t0")] = inp[key].clone()
+    elif wild:  # departure points anywhere within the halo, levels away
         g = torch.Generator(device="cuda").manual_seed(seed)
         for key, amp in (("uu_ext", 2.5 * cfg.dx), ("vv_ext", 2.5 * cfg.dx), ("ww_ext", 1500.0), ("ut0", 2.5 * cfg.dx),
                          ("vt0", 2.5 * cfg.dx), ("zdt0", 1500.0)):
+            amp = amp * float(wild)
             r = torch.rand(inp[key].shape, generator=g, device="cuda", dtype=torch.float64)
             inp[key] = ((2.0 * r - 1.0) * amp / cfg.dt).to(ft)
     return A, cfg, prec, ft, inp
@@ -40,7 +49,7 @@ def _bits(t):
 
 # niter 6 from the arrival points is the cold start
 @pytest.mark.parametrize("cold", [False, True])
-@pytest.mark.parametrize("wild", [False, True])
+@pytest.mark.parametrize("wild", [False, True, "shear"])
 @pytest.mark.parametrize("size", SIZES)
 @pytest.mark.parametrize("prec_name", ["mixed", "fp64"])
 def test_staged_step_equals_direct(prec_name, size, wild, cold):
@@ -131,6 +140,109 @@ def test_boundary_flux_shared_and_many():
     assert ad.status() == 0 and float(fi[0].abs().max()) > 0 and float(fo[0].abs().max()) > 0
     for q in range(len(srcs)):
         assert torch.equal(fo[q][m], go[q][m]) and torch.equal(fi[q][m], gi[q][m])
+
+
+# warm REF32 trajectories are staged from 56832 points on; scattered flows of
+# less amplitude than above, so that no stencil leaves the oracle's arrays
+@pytest.mark.parametrize("wild", [False, 0.5, "shear"])
+@pytest.mark.parametrize("size", [(33, 9, 5), (64, 40, 24), (97, 51, 13), (45, 300, 5), (40, 41, 60)])
+def test_staged_ref32_equals_oracle(size, wild):
+    from oracle import oracle as O
+    A, cfg, prec, ft, inp = _case("ref32", size, wild, 1)
+    st = O.Step(cfg, kind="oracle", prec="f32", lam=False)
+    np_in = {k: inp[k].cpu().numpy() for k in ("uu_ext", "vv_ext", "ww_ext", "ut0", "vt0", "zdt0")}
+    ad = A.Adz.from_config(cfg, lam=False)
+    px, wp = ad.new_state(prec)
+    st.inittraj()
+    ad.adz_inittraj(prec, px, wp)
+    for niter in (0, 1, 3):  # the first from the arrival points
+        st.traject(np_in, niter or None)
+        ad.adz_traject(prec, cfg.dt, inp, px, wp, niter=niter)
+        torch.cuda.synchronize()
+        assert ad.status() == 0
+        own = (slice(None), slice(None), slice(2, -2), slice(2, -2))
+        assert np.array_equal(px.cpu().numpy().view(np.int32), st.pxyzm.view(np.int32))
+        assert np.array_equal(wp.cpu().numpy()[own].view(np.int64), st.wpxyz[own].view(np.int64))
+
+
+@pytest.mark.parametrize("wild", [False, 0.5, "shear"])
+@pytest.mark.parametrize("size", [(33, 9, 5), (64, 40, 24), (97, 51, 13), (40, 41, 4), (31, 2, 8)])
+def test_tolerance_equals_fixed_updates(size, wild):
+    """The iteration to a tolerance (staged at every size) against fixed
+    updates of the direct kernel (small tiles): from the arrival points, from
+    stored points that converge at once, and with the fallback of a start that
+    does not; updates and counts."""
+    from gem_b200 import guess
+    A, cfg, prec, ft, inp = _case("mixed", size, wild, 1)
+    ad = A.Adz.from_config(cfg, lam=False)
+    n = cfg.ni * cfg.nj * cfg.nk
+    _, stored = ad.new_state(prec)
+    ad.adz_inittraj(prec, None, stored)
+    ad.adz_traject(prec, cfg.dt, inp, None, stored)
+
+    def run(tol, maxit, start):
+        wp = stored.clone()
+        it = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        st = torch.zeros(3, dtype=torch.int64, device="cuda")
+        guess.traject_tol(ad, prec, cfg.dt, inp, wp, tol=tol, maxit=maxit, start=start, iters=it, stats=st)
+        torch.cuda.synchronize()
+        return wp, it.cpu().numpy(), st.cpu().tolist()
+
+    def fixed(niter, cold):
+        wp = stored.clone()
+        if cold:
+            ad.adz_inittraj(prec, None, wp)
+        ad.adz_traject(prec, cfg.dt, inp, None, wp, niter=niter)
+        torch.cuda.synchronize()
+        return wp
+
+    own = (slice(None), slice(None), slice(2, -2), slice(2, -2))
+    # tolerance 0: a point stops where an update does not move it (further
+    # updates would not either), else it takes all of them
+    for tol, maxit, start, counts in ((0.0, 4, 0, [4 * n, 0, n]), (1e9, 3, 1, [n, 0, 0]), (0.0, 2, 1, [4 * n, n, n])):
+        wp, it, st = run(tol, maxit, start)
+        assert ad.status() == 0
+        back = torch.from_numpy(it >= 128).cuda().view(cfg.nk, cfg.nj, cfg.ni)
+        cold = fixed(maxit, True) if start == 0 or bool(back.any()) else wp
+        warm = fixed(1 if tol > 0.0 else maxit, False) if start == 1 else cold
+        assert ad.status() == 0
+        assert torch.equal(_bits(wp[own]), torch.where(back, _bits(cold[own]), _bits(warm[own])))
+        assert st[0] == int((it & 127).sum()) and st[1] == int(back.sum())
+        if wild == 0.5 or tol > 0.0:  # no point stops early
+            assert st == counts
+
+
+def test_more_rows_than_the_staged_grid():
+    """Above 131070 rows the grid of the staged kernels does not fit and the
+    direct ones run: the rows of a tile of 131100 against those of one of
+    131000, away from the upper edge."""
+    from gem_b200 import guess
+    A, cfg, prec, ft, big = _case("mixed", (8, 131100, 4), 0.5, 4)
+    rows = 130900
+    got = []
+    for nj in (131100, 131000):
+        cfg.nj = nj
+        njt = nj + 2 * cfg.halo
+        inp = {k: v[:, :njt].contiguous() for k, v in big.items() if k not in ("tracers", "uslt", "vslt")}
+        trs = [t[:, :njt].contiguous() for t in big["tracers"]]
+        ad = A.Adz.from_config(cfg, lam=False)
+        _, wp = ad.new_state(prec)
+        ad.adz_inittraj(prec, None, wp)
+        ad.adz_traject(prec, cfg.dt, inp, None, wp)
+        ad.adz_traject(prec, cfg.dt, inp, None, wp, niter=2)
+        out = [torch.zeros(ad.ext_shape, dtype=ft, device="cuda") for _ in range(8)]
+        ad.adz_tricub_hlt(prec, A.SET_T, trs, out[:4], mono=[1, 0, 1, 0])
+        ad.adz_tricub_hlt(prec, A.SET_T, trs, out[4:], mono=[A.QV | 1] * 4)
+        tol = wp.clone()
+        it = torch.zeros(cfg.ni * nj * cfg.nk, dtype=torch.uint8, device="cuda")
+        guess.traject_tol(ad, prec, cfg.dt, inp, tol, start=0, iters=it)
+        torch.cuda.synchronize()
+        assert ad.status() == 0
+        H = cfg.halo
+        got.append([w[:, :, 2:2 + rows, 2:-2] for w in (wp, tol)] + [o[:, H:H + rows] for o in out] +
+                   [it.view(cfg.nk, nj, cfg.ni)[:, :rows]])
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and float(a.double().abs().max()) > 0
 
 
 # REF32 starts from the stored FP32 positions as they are.  maxcfl 1 (halo 2):
