@@ -121,11 +121,12 @@ struct WindLayout {
 // offsets into the extended, the (ni,nj,nk) and the Adz_wpxyz arrays, in 32
 // bits (the first two volumes are below 2^31: adzc_setup refuses larger tiles)
 // or, I = long long, in 64.  The staged kernels take 32 bits (all in 64 bits:
-// MIXED step 2 % slower at 128 x 128 x 40, 4 % at 512 x 512 x 60).  The direct sets kernels
-// take 64, written out from ni and nj: ptxas then needs 80 registers instead
-// of 96 for FP64 and spills 16 bytes instead of 88 for REF32 (8 clipped
-// fields at 512 x 512 x 60 in REF32 3.27 ms, 3.70 in 32 bits; FP64 2 fields 1.28,
-// 1.37; MIXED 2 fields 0.816, 0.852)
+// MIXED step 2 % slower at 128 x 128 x 40, 4 % at 512 x 512 x 60).  The direct
+// sets kernels take 64, written out from ni and nj: ptxas then needs 80 registers
+// instead of 96 for FP64 and spills 16 bytes instead of 88 for REF32 (8 clipped
+// fields at 512 x 512 x 60 in REF32 3.28 ms, 3.67 in 32 bits; FP64 2 fields 1.28,
+// 1.36; MIXED 2 fields 0.816, 0.852).  k_tricub_parts of MIXED, u and v of
+// every step, takes 32 (3.61 ms at 1024 x 1024 x 80, 3.67 in 64)
 template <typename I = int>
 __device__ __forceinline__ long long ext_index(const DGrid& g, int i, int j, int k) {
   return (I)(i - g.lminx) + (I)(j - g.lminy) * g.nit + (k - 1) * (I)g.nij;
@@ -306,9 +307,10 @@ __device__ __forceinline__ double zindx_t(const DGrid& g, double posz) {
 }
 
 // stencil of a cell (ix local, x as in the ext array) stays inside the array
+template <typename I = int>
 __device__ __forceinline__ bool stencil_ok(const DGrid& g, int off) {
   // off = corner offset relative to cell (1,1,1): recover corner (i,j) in ext coords
-  const long long e = (long long)off + ext_index<long long>(g, 1, 1, 1);
+  const long long e = (long long)off + ext_index<I>(g, 1, 1, 1);
   const long long plane = g.nij;
   long long k = e >= 0 ? e / plane : -1;
   const long long r = e - k * plane;
@@ -788,7 +790,7 @@ __device__ __forceinline__ void set_point(const DGrid& g, int set, const SetArgs
   if (PREC == kMixed) {
     WF w;
     coef_mixed(w, px, py, pz, lv);
-    if (!stencil_ok(g, w.off)) { raise_status(g.status, kErrHalo); return; }
+    if (!stencil_ok<I>(g, w.off)) { raise_status(g.status, kErrHalo); return; }
     for (int q = 0; q < fp.nf; q++) {
       const float* f = (const float*)fp.src[q] + e111 + w.off;
       if (((fp.mono_mask >> q) & 1u) || PERT) {
@@ -811,7 +813,7 @@ __device__ __forceinline__ void set_point(const DGrid& g, int set, const SetArgs
     int off, zl;
     if (PREC == kRef32) zl = coef_f32pos(c, off, (float)px, (float)py, (float)pz, lv);
     else zl = coef_f64pos(c, off, px, py, pz, lv);
-    if (!stencil_ok(g, off)) { raise_status(g.status, kErrHalo); return; }
+    if (!stencil_ok<I>(g, off)) { raise_status(g.status, kErrHalo); return; }
     for (int q = 0; q < fp.nf; q++) {
       const F* f = (const F*)fp.src[q] + e111 + off;
       if (((fp.mono_mask >> q) & 1u) || PERT) {
@@ -910,7 +912,8 @@ __global__ void ADZ_PARTS_BOUNDS k_tricub_parts(DGrid g, SetArgs a, const __grid
   const int kk = (int)bk * TK + (int)((threadIdx.x / TI) % TK);
   const int jj = (int)(bj / nkg) * TJ + (int)(threadIdx.x / 128);
   if (ii >= P.nx || kk >= P.nz || jj >= P.ny) return;
-  set_point<PREC, false, PERT>(g, P.set, a, P.fp, ii + P.i0, jj + P.j0, kk + P.k0);
+  using I = typename std::conditional<PREC == kMixed, int, long long>::type;
+  set_point<PREC, false, PERT, I>(g, P.set, a, P.fp, ii + P.i0, jj + P.j0, kk + P.k0);
 #else
   const long long t = (long long)(blockIdx.x / (unsigned)sp.n) * blockDim.x + threadIdx.x;
   // points in (i, k, j) order, as in k_traject
@@ -1560,9 +1563,9 @@ cudaError_t launch_prepare_box(const DGrid& g, const void* uu, const void* vv, c
 template <int PREC>
 cudaError_t launch_traject_tol(const DGrid& g, const TrajArgs& a, double tol, int maxit, unsigned char* iters,
                                unsigned long long* stats, cudaStream_t s, const GuessStart& gs) {
-  // FP64 stays direct (not measured staged).  Rows that are no multiple of 16
-  // bytes gain less (first step of a run at 765 x 640 x 80: 10.33 ms staged, 10.62
-  // direct; 768: 8.76 and 9.65)
+  // FP64 is direct: the learned start, whose iteration this is, is MIXED only.
+  // Rows that are no multiple of 16 bytes gain less (first step of a run at 765 x
+  // 640 x 80: 10.33 ms staged, 10.62 direct; 768: 8.76 and 9.65)
   if constexpr (PREC == kMixed)
     if (st_traject_ok<PREC, true>(g, a, g.ni, g.nj))
       return st_launch_traject<PREC, true>(g, a, 1, g.ni, 1, g.nj, tol, maxit, iters, stats, gs, s);

@@ -104,6 +104,10 @@ constexpr int kStRing = 3;  // boxes in flight of the sets kernel
 // three (1024 x 512 x 80, 3 fields 4.13 and 3.89 ms, 4 4.79 and 4.91; 3 fields
 // without bounds 3.77 and 3.69, at 250 x 60 x 70 110 and 138 us).  The sets of REF32
 // stay direct (8 fields: 6.88 staged, 6.37 direct)
+// Rows that are no multiple of 16 bytes gain less (MIXED, 1021 x 512 x 80: 3 fields 2.41
+// ms staged, 2.63 direct, 5 3.68 and 4.18; BICUBH_QV at 637 x 512 x 80, 2 fields 1.57
+// and 1.95), and so does a single update of the trajectory (640 x 512 x 80: MIXED
+// 1.29 times as fast as direct, two updates 1.36; FP64 1.17, 1.40; REF32 1.04, 1.09)
 constexpr int kStQvMinFields = 2;
 template <int PREC>
 bool st_fields_ok(const FieldPtrs& fp) {
@@ -186,18 +190,23 @@ __device__ __forceinline__ StBox st_box(const DGrid& g, const int* red, int al) 
   }
   b.ox = (x1 - (x0 & ~(al - 1)) > C::RP ? imax_(x0, (x0 + x1 - C::RP) / 2) : x0) & ~(al - 1);
   b.nx = imin_(x1 - b.ox, C::RP);
+  if constexpr (!C::DYN) {
+    b.oy = y1 - y0 > C::BY ? (y0 + y1 - C::BY) / 2 : y0;
+    b.ny = imin_(y1 - b.oy, C::BY);
+    b.oz = z1 - z0 > C::BZ ? (z0 + z1 - C::BZ) / 2 : z0;
+    b.nz = imin_(z1 - b.oz, C::BZ);
+    b.pp = C::BY * C::RP;
+    return b;
+  }
   b.ny = y1 - y0;
   b.nz = z1 - z0;
-  if (!C::DYN) {
-    b.ny = imin_(b.ny, C::BY);
-    b.nz = imin_(b.nz, C::BZ);
-  } else if (b.ny * b.nz > C::ROWS) {  // BY rows, or those that the planes leave
+  if (b.ny * b.nz > C::ROWS) {  // BY rows, or those that the planes leave
     b.ny = imin_(b.ny, imax_(C::BY, C::ROWS / b.nz));
     b.nz = imin_(b.nz, C::ROWS / b.ny);
   }
-  b.pp = (C::DYN ? b.ny : C::BY) * C::RP;
   b.oy = (y0 + y1 - b.ny) / 2;
   b.oz = (z0 + z1 - b.nz) / 2;
+  b.pp = b.ny * C::RP;
   return b;
 }
 
