@@ -36,15 +36,18 @@
 // disjoint, so a sweep changes only its own shell and the centre), each
 // lane's cells stay in registers, and the list entry and bounds of a warp's
 // next tile are loaded before the barrier.  Bounds and cubes of 3 tracers at
-// 301 x 262 x 80, 3.4 % of the points outside: 20.4 ms with a launch per
-// wavefront (15 us each), 8.1 ms here (6 us).
+// 301 x 262 x 80, 3.4 % of the points outside, two sweeps: 20.4 ms with a launch
+// per wavefront (15 us each), 8.1 ms here (6 us).  1 % outside, one to four
+// sweeps: 8.1, 17.6, 39.0, 84.0 ms with launches, 4.3, 6.5, 8.9, 38.6 here (FP64 8.4,
+// 18.8, 43.3, 92.3 and 4.6, 6.5, 10.8, 58.9).  The values of four sweeps do not fit the
+// registers (552 bytes a lane in local memory, 960 in FP64): 30 % outside, 1024
+// x 512 x 80, FP64, took 704 ms with launches and takes 750.
 // Built with -fmad=false: the REAL arithmetic is the reference's, without
 // contraction.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "../../include/adz_b200.h"
 #include "adz_internal.h"
@@ -52,7 +55,6 @@
 
 namespace adz {
 namespace ilmc {
-
 
 struct Box {
   int il, ir, jl, jr, k0, nk;
@@ -65,12 +67,6 @@ struct Box {
 
 __device__ __forceinline__ long long ext(const Box& b, int i, int j, int k) {
   return (long long)(i - b.lminx) + (long long)(j - b.lminy) * b.nit + (long long)(k - 1) * b.nij;
-}
-
-__device__ __forceinline__ void coords(const Box& b, long long o, int& i, int& j, int& k) {
-  i = b.il + (int)(o % b.bx());
-  j = b.jl + (int)((o / b.bx()) % b.by());
-  k = b.k0 + (int)(o / ((long long)b.bx() * b.by()));
 }
 
 template <typename T>

@@ -1,8 +1,8 @@
 // MIXED instantiation: FP64 positions and cell offsets, FP32 weights and
 // packed FP32 sums.  Departure winds are stored as three component planes
 // (WindLayout in adz_kernels.cuh).  Block shapes and resident blocks per
-// SM of the direct kernels (adz_staged.cuh has the others) were picked by
-// timing the 1024x1024x80 step:
+// SM of the direct kernels (small launches, and the sets of one or two fields;
+// adz_staged.cuh has the others) were picked by timing the 1024x1024x80 step:
 //   trajectory  tiles of 32 i by 4 levels, 7 blocks of 128 threads: 9.54 ms
 //               (6, 8, 9 blocks: 9.84, 9.72, 10.42; 128 i of one level at
 //               8 blocks: 10.31 ms; 64 x 2: 10.00; 32 x 8 in blocks of 256
