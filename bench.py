@@ -397,7 +397,7 @@ def run_product(args):
                           "achieved_gbs": step_bytes / (ms32 * 1e-3) / 1e9,
                           "frac": step_bytes / (ms32 * 1e-3) / 1e9 / hbm},
         "accuracy": acc,
-        "e2e": e2e, "gpu_launches": (LAUNCHES_PER_STEP + (HALO_LAUNCHES_PER_STEP if ws > 1 else 0)) * args.steps,
+        "e2e": e2e, "gpu_launches": (mixed_step_launches(ad, args.ntr) + (HALO_LAUNCHES_PER_STEP if ws > 1 else 0)) * args.steps,
         "clocks": clk, "cpu_baseline": cpu,
         "tracers8": tsum, "post": psum, "batch": batch, "learned_guess": gsum, "level_a": lvla,
     }
@@ -542,9 +542,17 @@ def workload_config(args, ws, decomp=None):
             "points_per_step": ni * nj * nk, "l2": "inputs larger than L2 (no flush)", "parallelism": par}
 
 
-# kernels of one MIXED step: departure winds, trajectory, w with the tracers
-# from shared-memory boxes, and u and v in one direct launch
-LAUNCHES_PER_STEP = 4  # k_prepare4, k_traject_st, k_sets_st (three or more fields), k_tricub_parts
+def mixed_step_launches(ad, ntr):
+    """Kernels of one MIXED step: departure winds, trajectory and the sets, of
+    which w with the tracers takes a launch of its own where it is staged
+    (st_part_ok in adz_staged.cuh)."""
+    from gem_b200 import adz
+    i0, i1, j0, j1, k0 = ad.set_range(adz.SET_T)
+    n, nf = (i1 - i0 + 1) * (j1 - j0 + 1) * (ad.nk - k0 + 1), 1 + ntr
+    wave = 148 * 4 * 256  # points of the blocks that run at once
+    return 3 + (nf >= 3 and n * (2 if ad.info.nit % 4 == 0 else 1) >= wave and n * nf >= 4 * wave)
+
+
 HALO_LAUNCHES_PER_STEP = 4  # pack + unpack of the two exchanges (N > 1)
 
 
@@ -719,9 +727,7 @@ def measure_batch(args, timed, ws, cfgs, label):
             ad.adz_traject(prec, cfg.dt, inp, None, wp)
             ad.adz_tricub_sets(prec, [0, 1, 1, len(srcs) - 2], srcs, dsts, mono)
     ms_s, _ = timed(sequential, args.steps, args.warmup)
-    # per domain: winds, trajectory, u and v, and w with the tracers (a launch of
-    # its own from three fields on)
-    seq_launches = sum(3 + (1 + c.ntracers >= 3) for c in cfgs)
+    seq_launches = sum(mixed_step_launches(d[1], d[0].ntracers) for d in doms)
     plan = batch.query()
     nl = {"one launch": 1, "phased (one launch per phase)": 3}.get(plan["plan"], seq_launches)
     out = {"workload": f"{len(cfgs)} {label}",
