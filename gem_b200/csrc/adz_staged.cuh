@@ -103,11 +103,11 @@ constexpr int kStRing = 3;  // boxes in flight of the sets kernel
 // fields: 3.44 ms staged, 3.36 direct; 5 fields 5.64 and 7.19), in FP64 with bounds
 // three (1024 x 512 x 80, 3 fields 4.13 and 3.89 ms, 4 4.79 and 4.91; 3 fields
 // without bounds 3.77 and 3.69, at 250 x 60 x 70 110 and 138 us).  The sets of REF32
-// stay direct (8 fields: 6.88 staged, 6.37 direct)
-// Rows that are no multiple of 16 bytes gain less (MIXED, 1021 x 512 x 80: 3 fields 2.41
-// ms staged, 2.63 direct, 5 3.68 and 4.18; BICUBH_QV at 637 x 512 x 80, 2 fields 1.57
-// and 1.95), and so does a single update of the trajectory (640 x 512 x 80: MIXED
-// 1.29 times as fast as direct, two updates 1.36; FP64 1.17, 1.40; REF32 1.04, 1.09)
+// stay direct (8 fields: 6.88 staged, 6.37 direct).  Rows that are no
+// multiple of 16 bytes gain less (MIXED, 1021 x 512 x 80: 3 fields 2.41 ms staged,
+// 2.63 direct, 5 3.68 and 4.18; BICUBH_QV at 637 x 512 x 80, 2 fields 1.57 and 1.95),
+// and so does a single update of the trajectory (640 x 512 x 80: MIXED 1.29 times
+// as fast as direct, two updates 1.36; FP64 1.17, 1.40; REF32 1.04, 1.09)
 constexpr int kStQvMinFields = 2;
 template <int PREC>
 bool st_fields_ok(const FieldPtrs& fp) {

@@ -252,7 +252,8 @@ int adzc_bc_lam_zlf(adzc_handle *h, int prec, int setup, int ntr, void *const *f
  * Adz_j0b:jnb, 1:nk, then zeroed as the reference does (FLUX_out on the
  * core, FLUX_in on the pilot zones and above k0t); the fo, fi fields of
  * adzc_bermejo_conde.  srcs[q] NULL interpolates the masks themselves, the
- * PSADJ branch (:84-101).  The grid must set bc_lam_flux 1. */
+ * PSADJ branch (:84-101).  A tracer may lie in one of the call's fo, fi arrays:
+ * its values from before the call are used.  The grid must set bc_lam_flux 1. */
 int adzc_bc_lam_flux(adzc_handle *h, int prec, int ntr, const void *const *srcs, void *const *fo, void *const *fi,
                      void *stream);
 
